@@ -2,7 +2,7 @@
 
 Each translation unit is compiled by nvcc for ``sm_100a`` only and linked
 in-tree into ``particle_transport_b200/libptb200.so``.  ``push_exact.cu``,
-``lagstats.cu`` and ``init.cu`` are compiled with ``--fmad=false`` so that
+``lagstats.cu``, ``dmumu.cu`` and ``init.cu`` are compiled with ``--fmad=false`` so that
 the FP64 parity push, the mu reconstruction (also inside the fused
 phase-space binning), the statistics and the particle initialisation keep
 the reference's rounding (no fused multiply-add; explicit ``fma`` calls
@@ -28,6 +28,7 @@ UNITS = {
     "init.cu": ["--fmad=false"],
     "push_fast.cu": [],
     "lagstats.cu": ["--fmad=false"],
+    "dmumu.cu": ["--fmad=false"],
     "pt_api.cu": [],
     "pt_batch.cu": [],
     "hostio.cu": [],

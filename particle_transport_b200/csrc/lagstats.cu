@@ -1,20 +1,5 @@
 // Lag-pair statistics on the device.
 //
-// D_mumu / <dmu^2> (process_mu_chunk_dmumu_cpu!, src/compute_delta_mu2_dmumu_full.jl:457-704)
-// -----------------------------------------------------------------------------------------
-// Work unit = (particle, lag).  A warp owns one particle and 32 lags (lane =
-// lag); all lanes therefore visit the same start save s at the same time, and
-// the bin of a pair depends only on mu(s).  Each particle's mu series is
-// staged on chip together with the list of its valid start saves sorted
-// (stably) by start bin, so the pair loop runs bin by bin: every lane keeps
-// (count, sum dmu, sum dmu^2) for the current bin in registers and flushes
-// once per bin per particle into the CTA's shared (bin, lag) accumulators.
-// Per-particle <dmu^2> values feed per-lane Welford triples in registers.
-// CTA results go to per-CTA partials and a finalize kernel reduces them in
-// CTA order, merging Welford triples with the reference formula
-// (combine_welford_stats!, :439-455).  Integer counts are exact; FP64 sums
-// differ from the reference only by summation order.
-//
 // D_pp (process_momenta_chunk_dpp_cpu!, src/compute_dpp_full.jl:247-288)
 // ---------------------------------------------------------------------
 // Same layout without bins: |p| is computed once per (particle, save) in FP64
@@ -36,427 +21,6 @@ namespace pt {
 namespace {
 
 constexpr int kWarp = 32;
-constexpr int kStageWarps = 8;  // warps of a particle slot that stage its series
-
-struct WelfordPart {
-    long long count;
-    double mean, m2, pair_ss;
-    long long pair_n;
-};
-
-// combine_welford_stats! (src/compute_delta_mu2_dmumu_full.jl:439-455)
-__device__ __forceinline__ void welford_merge(long long& gc, double& gm, double& gm2, long long lc, double lm,
-                                              double lm2)
-{
-    if (lc <= 0) return;
-    if (gc == 0) {
-        gc = lc; gm = lm; gm2 = lm2;
-        return;
-    }
-    long long cc = gc + lc;
-    double delta = lm - gm;
-    gm += delta * (double)lc / (double)cc;
-    gm2 += lm2 + delta * delta * (double)gc * (double)lc / (double)cc;
-    gc = cc;
-}
-
-// mu_bin_value + mu_bin_index_full (dmumu:304-318): 0-based bin, n_bins for a
-// finite value outside [edges[0], edges[n_bins]], -1 for a non-finite value.
-// searchsortedlast (the last edge <= v) is found from a guess on a uniform
-// grid, inv_w = n_bins / (edges[n_bins] - edges[0]), moved up and down until
-// edges[b] <= v < edges[b + 1]: the same bin as a binary search over the
-// stored Float64 edges for any increasing edges, in one or two compares for
-// the uniform edges of build_mu_edges_full (a range).
-__device__ __forceinline__ int bin_of(double v, const double* __restrict__ edges, int n_bins, int bin_abs,
-                                      double inv_w)
-{
-    if (!isfinite(v)) return -1;
-    if (bin_abs) v = fabs(v);
-    if (v < edges[0] || v > edges[n_bins]) return n_bins;
-    int b = (int)fmin(fmax((v - edges[0]) * inv_w, 0.0), (double)(n_bins - 1));
-    while (b < n_bins && edges[b + 1] <= v) ++b;
-    while (b > 0 && edges[b] > v) --b;
-    return b == n_bins ? n_bins - 1 : b;  // v == edges[n_bins] falls in the last bin
-}
-
-struct DmumuLaunch {
-    int64_t n, nsave;
-    int64_t start_cap;         // 1 for the injection estimator, nsave for sliding
-    const int64_t* lags;       // this batch's lags
-    int nl;                    // lags in this batch
-    const double* edges;
-    int n_bins, bin_abs;
-    int ppc, groups;           // particle slots per CTA, 32-lag groups per slot
-    int parts;                 // warps splitting the bins of one (slot, lag group)
-    size_t slot_bytes;
-    char* gslots;              // global staging when the slots do not fit on chip
-    // per-CTA outputs
-    unsigned long long* part_cnt;  // [grid][nl][n_bins]
-    double* part_sd;
-    double* part_sd2;
-    WelfordPart* part_w;           // [grid][nl]
-};
-
-// Where dmumu_kernel reads the mu series of particle p: a mu chunk at the
-// compute precision T (the reference's mu_chunk, Float32 by default), element
-// (p, s) at p * sp + s * ss.
-template <typename T_>
-struct CacheSourceT {
-    using T = T_;
-    const T_* mu;
-    int64_t sp, ss;
-    __device__ __forceinline__ T_ operator()(int64_t p, int64_t s) const { return mu[p * sp + s * ss]; }
-};
-using CacheSource = CacheSourceT<float>;
-// bytes of one particle slot of dmumu_kernel (layout in the kernel)
-size_t dmumu_slot_bytes(int64_t nsave, size_t mu_bytes, size_t idx_bytes, int n_bins, int nl_cap)
-{
-    auto a16 = [](size_t v) { return (v + 15) & ~(size_t)15; };
-    return a16((size_t)(nsave + 1) * mu_bytes) + a16((size_t)nsave * idx_bytes) +
-           a16(sizeof(int) * (size_t)(kStageWarps * (n_bins + 1) + n_bins + 2)) + a16(16 * (size_t)nl_cap);
-}
-
-template <typename IdxT, bool SMEM_SLOTS, class Src>
-__global__ void __launch_bounds__(1024) dmumu_kernel(DmumuLaunch a, Src source)
-{
-    using MuT = typename Src::T;
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int nb = a.n_bins, nl = a.nl;
-    // shared layout: edges | acc_cnt | acc_sd | acc_sd2 ([bin][lag] each) | slots
-    double* s_edges = (double*)smem;
-    size_t off = ((size_t)(nb + 1) * sizeof(double) + 15) & ~(size_t)15;
-    unsigned long long* acc_cnt = (unsigned long long*)(smem + off);
-    off += (size_t)nl * nb * sizeof(unsigned long long);
-    double* acc_sd = (double*)(smem + off);
-    off += (size_t)nl * nb * sizeof(double);
-    double* acc_sd2 = (double*)(smem + off);
-    off += (size_t)nl * nb * sizeof(double);
-    unsigned char* slot_base = SMEM_SLOTS ? (smem + off) : (unsigned char*)(a.gslots + (size_t)blockIdx.x * a.ppc * a.slot_bytes);
-
-    for (int i = threadIdx.x; i <= nb; i += blockDim.x) s_edges[i] = a.edges[i];
-    const double span = a.edges[nb] - a.edges[0];
-    const double inv_w = span > 0.0 && isfinite(span) ? (double)nb / span : 0.0;
-    for (int i = threadIdx.x; i < nl * nb; i += blockDim.x) {
-        acc_cnt[i] = 0ull;
-        acc_sd[i] = 0.0;
-        acc_sd2[i] = 0.0;
-    }
-
-    // Lags are dealt to the 32-lane groups so that lags equal modulo 32 --
-    // which read the same shared-memory bank at every start -- fall into
-    // different groups where possible.  s_lane_lag[g*32 + lane] = lag index
-    // (-1: idle lane), s_lag_pos[lag] = g*32 + lane.
-    __shared__ int s_lane_lag[8 * kWarp];
-    __shared__ int s_lag_pos[8 * kWarp];
-    __shared__ unsigned char cnt[8][kWarp];
-    __shared__ int fill[8];
-    for (int i = threadIdx.x; i < 8 * kWarp; i += blockDim.x) {
-        s_lane_lag[i] = -1;
-        cnt[i / kWarp][i % kWarp] = 0;
-    }
-    if (threadIdx.x < 8) fill[threadIdx.x] = 0;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < nl; ++i) {
-            const int r = (int)(((a.lags[i] % kWarp) + kWarp) % kWarp);
-            int best = -1;
-            for (int g = 0; g < a.groups; ++g) {
-                if (fill[g] >= kWarp) continue;
-                if (best < 0 || cnt[g][r] < cnt[best][r] || (cnt[g][r] == cnt[best][r] && fill[g] < fill[best]))
-                    best = g;
-            }
-            const int pos = best * kWarp + fill[best]++;
-            cnt[best][r]++;
-            s_lane_lag[pos] = i;
-            s_lag_pos[i] = pos;
-        }
-    }
-    __syncthreads();
-
-    const int warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
-    const int wps = a.groups * a.parts;  // warps per particle slot
-    const int slot = warp / wps, group = (warp % wps) / a.parts, part = warp % a.parts;
-    const int li = s_lane_lag[group * kWarp + lane];
-    const bool lane_on = li >= 0;
-    int64_t L = lane_on ? a.lags[li] : 0;
-    if (L < 1 || L >= a.nsave) L = a.nsave;  // reference: lag >= nsteps -> skipped (valid starts: s < nsave - L)
-
-    // slot layout: series[nsave + 1] MuT | list[nsave] IdxT | whist[kStageWarps][nb+1] int
-    //              | cur[nb+2] int | tot_c[nl] u64 | tot_sd2[nl] f64 (per-particle totals over the bins)
-    // The series holds the finite mu values and NaN for the others, and
-    // series[nsave] = NaN: a lag partner past the end of the series reads it.
-    unsigned char* sb = slot_base + (size_t)slot * a.slot_bytes;
-    MuT* series = (MuT*)sb;
-    IdxT* list = (IdxT*)(sb + (((a.nsave + 1) * sizeof(MuT) + 15) & ~(size_t)15));
-    int* whist = (int*)((unsigned char*)list + ((a.nsave * sizeof(IdxT) + 15) & ~(size_t)15));
-    int* cur = whist + kStageWarps * (nb + 1);
-    unsigned long long* tot_c = (unsigned long long*)((unsigned char*)whist +
-                                                      ((sizeof(int) * (size_t)(kStageWarps * (nb + 1) + nb + 2) + 15) &
-                                                       ~(size_t)15));
-    double* tot_sd2 = (double*)(tot_c + nl);
-    // staging is shared by the first `stagers` warps of the slot, each taking a
-    // contiguous range of saves; per-warp bin counts, offset in warp order,
-    // give the same bin-sorted start list (ascending starts within a bin)
-    // as a single warp walking the series
-    const int wis = warp % wps;
-    const int stagers = min(wps, kStageWarps);
-
-    long long wc = 0, pn = 0;
-    double wm = 0.0, wm2 = 0.0, pss = 0.0;
-    const int64_t scap = min(a.start_cap, a.nsave);
-    const unsigned lt_mask = (1u << lane) - 1u;
-
-    __syncthreads();
-    const int64_t tiles = (a.n + a.ppc - 1) / a.ppc;
-    for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const int64_t p = tile * a.ppc + slot;
-        const bool have = p < a.n;
-        // ---- stage: series, per-warp bin counts
-        if (have && wis < stagers) {
-            const int64_t per = ((a.nsave + stagers - 1) / stagers + kWarp - 1) / kWarp * kWarp;
-            const int64_t st_begin = (int64_t)wis * per, st_end = min(a.nsave, st_begin + per);
-            int* my_hist = whist + wis * (nb + 1);
-            for (int b = lane; b <= nb; b += kWarp) my_hist[b] = 0;
-            if (wis == 0) {
-                for (int l = lane; l < nl; l += kWarp) {
-                    tot_c[l] = 0ull;
-                    tot_sd2[l] = 0.0;
-                }
-                if (lane == 0) series[a.nsave] = MuT(NAN);
-            }
-            __syncwarp();
-            for (int64_t s0 = st_begin; s0 < st_end; s0 += kWarp) {
-                const int64_t s = s0 + lane;
-                int b = -1;
-                if (s < st_end) {
-                    const MuT v = source(p, s);
-                    series[s] = isfinite(v) ? v : MuT(NAN);
-                    if (s < scap) b = bin_of((double)v, s_edges, nb, a.bin_abs, inv_w);
-                }
-                const unsigned active = __ballot_sync(0xffffffffu, b >= 0);
-                if (b >= 0) {
-                    const unsigned same = __match_any_sync(active, b);
-                    if ((same & lt_mask) == 0) my_hist[b] += __popc(same);
-                }
-                __syncwarp();
-            }
-        }
-        __syncthreads();
-        // ---- offsets: bin-major, then stager order within a bin
-        if (have && wis == 0) {
-            int carry = 0;
-            for (int b0 = 0; b0 <= nb; b0 += kWarp) {
-                const int b = b0 + lane;
-                int t = 0;
-                if (b <= nb)
-                    for (int w = 0; w < stagers; ++w) t += whist[w * (nb + 1) + b];
-                int incl = t;
-                for (int d = 1; d < kWarp; d <<= 1) {
-                    const int y = __shfl_up_sync(0xffffffffu, incl, d);
-                    if (lane >= d) incl += y;
-                }
-                if (b <= nb) {
-                    int run = carry + incl - t;
-                    cur[b] = run;
-                    for (int w = 0; w < stagers; ++w) {
-                        const int c = whist[w * (nb + 1) + b];
-                        whist[w * (nb + 1) + b] = run;
-                        run += c;
-                    }
-                }
-                carry += __shfl_sync(0xffffffffu, incl, kWarp - 1);
-            }
-            if (lane == 0) cur[nb + 1] = carry;
-        }
-        __syncthreads();
-        // ---- scatter each stager's starts in order
-        if (have && wis < stagers) {
-            const int64_t per = ((a.nsave + stagers - 1) / stagers + kWarp - 1) / kWarp * kWarp;
-            const int64_t st_begin = (int64_t)wis * per, st_end = min(a.nsave, st_begin + per);
-            int* my_hist = whist + wis * (nb + 1);
-            const int64_t end = min(st_end, scap);
-            for (int64_t s0 = st_begin; s0 < end; s0 += kWarp) {
-                const int64_t s = s0 + lane;
-                int b = -1;
-                if (s < end) b = bin_of((double)series[s], s_edges, nb, a.bin_abs, inv_w);
-                const unsigned active = __ballot_sync(0xffffffffu, b >= 0);
-                if (b >= 0) {
-                    const unsigned same = __match_any_sync(active, b);
-                    const int rank = __popc(same & lt_mask);
-                    list[my_hist[b] + rank] = (IdxT)s;
-                    __syncwarp(active);
-                    if (rank == 0) my_hist[b] += __popc(same);
-                }
-                __syncwarp();
-            }
-        }
-        __syncthreads();
-        // ---- pairs: the `parts` warps of a (slot, lag group) split the
-        // bin-sorted start list into equal shares (a bin may straddle two
-        // shares; each flushes its part of it), so they reach the barrier
-        // together whatever the particle's bin counts; every lane keeps two
-        // accumulator chains
-        if (have) {
-            long long my_c = 0;
-            double my_sd2 = 0.0;
-            // starts, lags and nsave fit 32 bits (nsave < 2^31); so does a bin's count
-            const unsigned n32 = (unsigned)a.nsave, L32 = (unsigned)L;
-            const int total = cur[nb + 1];
-            const int r0 = (int)(((long long)total * part) / a.parts);
-            const int r1 = (int)(((long long)total * (part + 1)) / a.parts);
-            int b = 0;
-            if (r0 < r1)
-                while (cur[b + 1] <= r0) ++b;  // the bin holding entry r0 (r0 < total = cur[nb + 1])
-            for (int e = r0; e < r1; ++b) {
-                const int e1 = min(cur[b + 1], r1);
-                int c = 0;
-                double sd0 = 0.0, sd1 = 0.0, sq0 = 0.0, sq1 = 0.0;
-                // Branch-free pairs.  A start in the list has a finite mu; its
-                // partner series[s + L] is NaN when the particle's mu is not
-                // finite there, and s + L past the series end reads the NaN pad
-                // (idle lanes have L = nsave).  An invalid partner is replaced by
-                // the start's own value, so the pair adds +0 and 0 * 0 -- the
-                // sums are bit-identical to skipping it (they are never -0).
-                for (; e + 4 <= e1; e += 4) {
-                    MuT a_[4], v_[4];
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const unsigned s = (unsigned)list[e + k];
-                        a_[k] = series[s];
-                        v_[k] = series[min(s + L32, n32)];
-                    }
-#pragma unroll
-                    for (int k = 0; k < 4; k += 2) {
-                        const bool ok0 = v_[k] == v_[k], ok1 = v_[k + 1] == v_[k + 1];
-                        const MuT w0 = ok0 ? v_[k] : a_[k], w1 = ok1 ? v_[k + 1] : a_[k + 1];
-                        c += (int)ok0 + (int)ok1;
-                        const double d0 = (double)w0 - (double)a_[k];
-                        const double d1 = (double)w1 - (double)a_[k + 1];
-                        sd0 += d0;
-                        sq0 = fma(d0, d0, sq0);
-                        sd1 += d1;
-                        sq1 = fma(d1, d1, sq1);
-                    }
-                }
-                for (; e < e1; ++e) {
-                    const unsigned s = (unsigned)list[e];
-                    const MuT av = series[s];
-                    const MuT vv = series[min(s + L32, n32)];
-                    const bool ok = vv == vv;
-                    const double d = (double)(ok ? vv : av) - (double)av;
-                    c += (int)ok;
-                    sd0 += d;
-                    sq0 = fma(d, d, sq0);
-                }
-                const double sd = sd0 + sd1, sd2 = sq0 + sq1;
-                if (b < nb && c > 0 && lane_on) {
-                    const int ai = b * nl + li;  // [bin][lag]: the lanes of a flush hit consecutive words
-                    atomicAdd(&acc_cnt[ai], (unsigned long long)c);
-                    atomicAdd(&acc_sd[ai], sd);
-                    atomicAdd(&acc_sd2[ai], sd2);
-                }
-                my_c += c;
-                my_sd2 += sd2;
-                e = e1;
-            }
-            if (lane_on && my_c > 0) {
-                atomicAdd(&tot_c[li], (unsigned long long)my_c);
-                atomicAdd(&tot_sd2[li], my_sd2);
-            }
-        }
-        __syncthreads();
-        if (have && part == 0 && lane_on) {
-            const long long tc = (long long)tot_c[li];
-            const double ts = tot_sd2[li];
-            if (tc > 0) {
-                // per-particle value: mean dmu^2 over its valid pairs (dmumu:528-537);
-                // for the injection estimator tc == 1 and the value is dmu^2 (:625-631)
-                const double value = ts / (double)tc;
-                wc += 1;
-                const double delta = value - wm;
-                wm += delta / (double)wc;
-                wm2 += delta * (value - wm);
-                pss += ts;
-                pn += tc;
-            }
-        }
-        __syncthreads();
-    }
-
-    // ---- CTA epilogue: (bin, lag) accumulators and Welford triples
-    const int64_t cta = blockIdx.x;
-    for (int i = threadIdx.x; i < nl * nb; i += blockDim.x) {
-        const int j = (i % nb) * nl + i / nb;  // partials are [lag][bin], the shared sums [bin][lag]
-        a.part_cnt[cta * nl * nb + i] = acc_cnt[j];
-        a.part_sd[cta * nl * nb + i] = acc_sd[j];
-        a.part_sd2[cta * nl * nb + i] = acc_sd2[j];
-    }
-    __syncthreads();
-    // reuse the accumulator region to gather per-warp Welford triples
-    WelfordPart* wp = (WelfordPart*)(smem + (((size_t)(nb + 1) * sizeof(double) + 15) & ~(size_t)15));
-    const int nwarps = blockDim.x / kWarp;
-    wp[warp * kWarp + lane] = WelfordPart{wc, wm, wm2, pss, pn};
-    __syncthreads();
-    for (int l = threadIdx.x; l < nl; l += blockDim.x) {
-        const int g = s_lag_pos[l] / kWarp, ln = s_lag_pos[l] % kWarp;
-        long long c = 0, n2 = 0;
-        double m = 0.0, m2 = 0.0, ss = 0.0;
-        for (int sl = 0; sl < a.ppc; ++sl) {
-            const int w = sl * wps + g * a.parts;  // the part-0 warp holds the slot's Welford triple
-            if (w >= nwarps) break;
-            const WelfordPart q = wp[w * kWarp + ln];
-            welford_merge(c, m, m2, q.count, q.mean, q.m2);
-            ss += q.pair_ss;
-            n2 += q.pair_n;
-        }
-        a.part_w[cta * nl + l] = WelfordPart{c, m, m2, ss, n2};
-    }
-}
-
-// Reduce per-CTA partials in CTA order and add / merge into the outputs.
-__global__ void dmumu_finalize_kernel(const unsigned long long* __restrict__ part_cnt,
-                                      const double* __restrict__ part_sd, const double* __restrict__ part_sd2,
-                                      const WelfordPart* __restrict__ part_w, int grid, int nl, int nb, int lag0,
-                                      int n_lags_total, int64_t* counts, double* sum_d, double* sum_d2,
-                                      int64_t* w_count, double* w_mean, double* w_m2, double* pair_ss,
-                                      int64_t* pair_n)
-{
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < nl * nb) {
-        unsigned long long c = 0;
-        double sd = 0.0, sd2 = 0.0;
-        for (int g = 0; g < grid; ++g) {
-            c += part_cnt[(int64_t)g * nl * nb + t];
-            sd += part_sd[(int64_t)g * nl * nb + t];
-            sd2 += part_sd2[(int64_t)g * nl * nb + t];
-        }
-        const int l = t / nb, b = t % nb;
-        const int64_t o = (int64_t)(lag0 + l) * nb + b;  // Julia (n_bins, n_lags)
-        counts[o] += (int64_t)c;
-        sum_d[o] += sd;
-        sum_d2[o] += sd2;
-    }
-    if (t < nl) {
-        long long c = 0, n2 = 0;
-        double m = 0.0, m2 = 0.0, ss = 0.0;
-        for (int g = 0; g < grid; ++g) {
-            const WelfordPart q = part_w[(int64_t)g * nl + t];
-            welford_merge(c, m, m2, q.count, q.mean, q.m2);
-            ss += q.pair_ss;
-            n2 += q.pair_n;
-        }
-        const int l = lag0 + t;
-        long long gc = w_count[l];
-        double gm = w_mean[l], gm2 = w_m2[l];
-        welford_merge(gc, gm, gm2, c, m, m2);
-        w_count[l] = gc;
-        w_mean[l] = gm;
-        w_m2[l] = gm2;
-        pair_ss[l] += ss;
-        pair_n[l] += n2;
-    }
-    (void)n_lags_total;
-}
 
 // ------------------------------------------------------------------ D_pp
 // momentum_magnitude (src/compute_dpp_full.jl:232-234) with the reference's
@@ -669,119 +233,6 @@ __global__ void energy_hist_kernel(const float* __restrict__ mom, int64_t chunk,
 
 size_t align16(size_t b) { return (b + 15) & ~(size_t)15; }
 
-// Particle slots per CTA (ppc <= max_ppc) and warps per (slot, lag group)
-// (parts): the most warps per CTA (at most 32), the larger ppc among equals.
-// With 55 lags (two groups) and room for five slots this gives 4 slots x 4
-// parts, 32 warps: 8.58e11 lag-pairs/s against 8.28e11 for 5 x 3 (30 warps).
-constexpr int kMaxParts = 8;
-void dmumu_shape(int max_ppc, int groups, int& ppc, int& parts)
-{
-    int best = 0;
-    ppc = 1;
-    parts = 1;
-    for (int c = 1; c <= std::max(1, max_ppc) && c * groups <= 32; ++c) {
-        const int pt = std::max(1, std::min(kMaxParts, 32 / (c * groups)));
-        if (c * groups * pt >= best) {
-            best = c * groups * pt;
-            ppc = c;
-            parts = pt;
-        }
-    }
-}
-
-}  // namespace
-
-// ------------------------------------------------------------------ host side
-namespace {
-
-// D_mumu over the series that `src` yields (a.mu, a.sp, a.ss are not used here)
-template <class Src>
-int run_dmumu_src(pt_ctx* ctx, const DmumuArgs& a, const Src& src, cudaStream_t s)
-{
-    using MuT = typename Src::T;
-    if (a.n <= 0 || a.n_lags <= 0) return PT_OK;
-    if (a.n_bins < 1 || a.n_bins > 4096) return fail(PT_ERR_ARG, "n_bins must be in [1, 4096]");
-    if (a.nsave < 1) return fail(PT_ERR_ARG, "nsave must be positive");
-    int dev = ctx->device;
-    int max_smem = 0;
-    cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    const size_t budget = (size_t)std::min(max_smem, 200 * 1024);
-    const bool small_idx = a.nsave <= 65535;
-    const size_t idx_bytes = small_idx ? 2 : 4;
-    const size_t edge_bytes = align16(sizeof(double) * (size_t)(a.n_bins + 1));
-    // lags per launch: multiple of 32 with the accumulators taking <= ~half the budget
-    int nl_cap = (int)std::max<size_t>(32, ((budget / 2) / ((size_t)a.n_bins * 24)) / 32 * 32);
-    nl_cap = std::min(nl_cap, 32 * 8);
-    const size_t slot_bytes = dmumu_slot_bytes(a.nsave, sizeof(MuT), idx_bytes, a.n_bins, nl_cap);
-    const int lag_batches = (a.n_lags + nl_cap - 1) / nl_cap;
-    for (int lb = 0; lb < lag_batches; ++lb) {
-        const int lag0 = lb * nl_cap;
-        const int nl = std::min(nl_cap, a.n_lags - lag0);
-        const int groups = (nl + kWarp - 1) / kWarp;
-        const size_t acc_bytes = (size_t)nl * a.n_bins * 24;
-        size_t fixed = edge_bytes + std::max(acc_bytes, sizeof(WelfordPart) * 1024);
-        bool smem_slots = fixed + slot_bytes <= budget;
-        // more warps share each staged series: its start list is split over `parts` warps
-        int ppc, parts;
-        dmumu_shape(smem_slots ? (int)std::min<size_t>((budget - fixed) / slot_bytes, 32) : 8, groups, ppc, parts);
-        const int threads = ppc * groups * parts * kWarp;
-        size_t smem = fixed + (smem_slots ? (size_t)ppc * slot_bytes : 0);
-        const int64_t tiles = (a.n + ppc - 1) / ppc;
-        int per_sm = 1;
-        void* kfn = small_idx ? (smem_slots ? (void*)dmumu_kernel<uint16_t, true, Src>
-                                           : (void*)dmumu_kernel<uint16_t, false, Src>)
-                              : (smem_slots ? (void*)dmumu_kernel<uint32_t, true, Src>
-                                            : (void*)dmumu_kernel<uint32_t, false, Src>);
-        PT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, threads, smem);
-        per_sm = std::max(1, per_sm);
-        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)ctx->num_sms * per_sm));
-        // scratch: per-CTA partials (+ global staging slots when needed)
-        const size_t part_acc = (size_t)grid * nl * a.n_bins;
-        const size_t bytes = align16(part_acc * 8) * 3 + align16(sizeof(WelfordPart) * (size_t)grid * nl) +
-                             (smem_slots ? 0 : (size_t)grid * ppc * slot_bytes);
-        void* scratch = nullptr;
-        int rc = scratch_get(ctx, 0, bytes, &scratch);
-        if (rc) return rc;
-        char* base = (char*)scratch;
-        DmumuLaunch L;
-        L.n = a.n; L.nsave = a.nsave;
-        L.start_cap = a.injection ? 1 : a.nsave;
-        L.lags = a.lags + lag0; L.nl = nl; L.edges = a.edges; L.n_bins = a.n_bins; L.bin_abs = a.bin_abs;
-        L.ppc = ppc; L.groups = groups; L.parts = parts; L.slot_bytes = slot_bytes;
-        L.part_cnt = (unsigned long long*)base;
-        L.part_sd = (double*)(base + align16(part_acc * 8));
-        L.part_sd2 = (double*)(base + 2 * align16(part_acc * 8));
-        L.part_w = (WelfordPart*)(base + 3 * align16(part_acc * 8));
-        L.gslots = smem_slots ? nullptr : (char*)L.part_w + align16(sizeof(WelfordPart) * (size_t)grid * nl);
-        if (small_idx) {
-            if (smem_slots) dmumu_kernel<uint16_t, true, Src><<<grid, threads, smem, s>>>(L, src);
-            else dmumu_kernel<uint16_t, false, Src><<<grid, threads, smem, s>>>(L, src);
-        } else {
-            if (smem_slots) dmumu_kernel<uint32_t, true, Src><<<grid, threads, smem, s>>>(L, src);
-            else dmumu_kernel<uint32_t, false, Src><<<grid, threads, smem, s>>>(L, src);
-        }
-        PT_CHECK_LAUNCH("dmumu_kernel");
-        const int fin_threads = 256;
-        const int fin_blocks = (int)((std::max(nl * a.n_bins, nl) + fin_threads - 1) / fin_threads);
-        dmumu_finalize_kernel<<<fin_blocks, fin_threads, 0, s>>>(L.part_cnt, L.part_sd, L.part_sd2, L.part_w, grid, nl,
-                                                                 a.n_bins, lag0, a.n_lags, a.counts, a.sum_d,
-                                                                 a.sum_d2, a.w_count, a.w_mean, a.w_m2, a.pair_ss,
-                                                                 a.pair_n);
-        PT_CHECK_LAUNCH("dmumu_finalize_kernel");
-    }
-    return PT_OK;
-}
-
-}  // namespace
-
-int run_dmumu(pt_ctx* ctx, const DmumuArgs& a, cudaStream_t s)
-{
-    return run_dmumu_src(ctx, a, CacheSource{a.mu, a.sp, a.ss}, s);
-}
-
-namespace {
-
 // (Bx, By, Bz) column-major arrays -> one record per node
 template <typename R>
 __global__ void interleave_b_kernel(const R* __restrict__ bx, const R* __restrict__ by, const R* __restrict__ bz,
@@ -893,7 +344,7 @@ int run_dmumu_phase_space_t(pt_ctx* ctx, const DmumuArgs& a, const R* pos, const
         PT_CHECK_LAUNCH("phase_space_mu_kernel");
         DmumuArgs c = a;
         c.n = m;
-        rc = run_dmumu_src(ctx, c, CacheSourceT<R>{mu, 1, m}, s);
+        rc = run_dmumu_chunk(ctx, c, mu, 1, m, sizeof(R) == 8, s);
         if (rc) return rc;
     }
     return PT_OK;
@@ -997,147 +448,3 @@ int launch_energy_histogram(const float* mom, int64_t chunk, int64_t nsave, cons
 }
 
 }  // namespace pt
-
-// ---------------------------------------------------------------------------
-// D_mumu accumulation that allocates nothing.
-//
-// Some callers cannot let a library allocate device memory: a host that owns
-// all device memory through its own pool (the Julia host's CUDA.jl pool, or
-// the campaign server's HBM-budget admission) has no way to account for a
-// cudaMalloc made behind its back, and cudaFree synchronises the whole
-// device, stalling every other stream of a busy GPU.  For them the per-CTA
-// partials of the D_mumu kernel live in a fixed, file-scope device array of
-// kDmumuNoAllocBytes (16 MiB) that every GPU which loads the library holds
-// until the process exits.  The array's device address is looked up once per
-// device with cudaGetSymbolAddress (host code cannot use the symbol itself:
-// on the host it names a stand-in, not device memory).
-// ---------------------------------------------------------------------------
-#include <mutex>
-
-static constexpr size_t kDmumuNoAllocBytes = (size_t)16 << 20;
-static __device__ __align__(256) unsigned char g_dmumu_noalloc_scratch[kDmumuNoAllocBytes];
-
-namespace pt {
-namespace {
-
-constexpr int kMaxDevices = 64;
-std::mutex g_noalloc_mutex;
-void* g_noalloc_ptr[kMaxDevices] = {};
-
-// Device address of the fixed scratch on `device` (set up on first use).
-int noalloc_scratch(int device, void** out)
-{
-    if (device < 0 || device >= kMaxDevices) return fail(PT_ERR_ARG, "device index out of range");
-    std::lock_guard<std::mutex> lock(g_noalloc_mutex);
-    if (!g_noalloc_ptr[device]) {
-        int prev = 0;
-        cudaError_t e = cudaGetDevice(&prev);
-        if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
-        e = cudaSetDevice(device);
-        if (e != cudaSuccess) return cuda_fail(e, "cudaSetDevice");
-        void* p = nullptr;
-        e = cudaGetSymbolAddress(&p, g_dmumu_noalloc_scratch);
-        cudaError_t e2 = cudaSetDevice(prev);
-        if (e != cudaSuccess) return cuda_fail(e, "cudaGetSymbolAddress(g_dmumu_noalloc_scratch)");
-        if (e2 != cudaSuccess) return cuda_fail(e2, "cudaSetDevice");
-        g_noalloc_ptr[device] = p;
-    }
-    *out = g_noalloc_ptr[device];
-    return PT_OK;
-}
-
-int run_dmumu_noalloc(pt_ctx* ctx, const DmumuArgs& a, cudaStream_t s)
-{
-    if (a.n <= 0 || a.n_lags <= 0) return PT_OK;
-    if (a.n_bins < 1 || a.n_bins > 4096) return fail(PT_ERR_ARG, "n_bins must be in [1, 4096]");
-    if (a.nsave < 1) return fail(PT_ERR_ARG, "nsave must be positive");
-    void* scratch = nullptr;
-    int rc = noalloc_scratch(ctx->device, &scratch);
-    if (rc) return rc;
-    int max_smem = 0;
-    cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
-    const size_t budget = (size_t)std::min(max_smem, 200 * 1024);
-    const bool small_idx = a.nsave <= 65535;
-    const size_t idx_bytes = small_idx ? 2 : 4;
-    const size_t edge_bytes = align16(sizeof(double) * (size_t)(a.n_bins + 1));
-    int nl_cap = (int)std::max<size_t>(32, ((budget / 2) / ((size_t)a.n_bins * 24)) / 32 * 32);
-    nl_cap = std::min(nl_cap, 32 * 8);
-    const size_t slot_bytes = dmumu_slot_bytes(a.nsave, sizeof(float), idx_bytes, a.n_bins, nl_cap);
-    const CacheSource src{a.mu, a.sp, a.ss};
-    for (int lag0 = 0; lag0 < a.n_lags; lag0 += nl_cap) {
-        const int nl = std::min(nl_cap, a.n_lags - lag0);
-        const int groups = (nl + kWarp - 1) / kWarp;
-        const size_t acc_bytes = (size_t)nl * a.n_bins * 24;
-        const size_t fixed = edge_bytes + std::max(acc_bytes, sizeof(WelfordPart) * 1024);
-        if (fixed + slot_bytes > budget)
-            return fail(PT_ERR_ARG, "pt_dmumu_accumulate_device_noalloc: nsave = " + std::to_string(a.nsave) +
-                                        " is too long for on-chip staging with " + std::to_string(a.n_bins) +
-                                        " bins; use pt_dmumu_accumulate_device");
-        int ppc, parts;
-        dmumu_shape((int)std::min<size_t>((budget - fixed) / slot_bytes, 32), groups, ppc, parts);
-        const int threads = ppc * groups * parts * kWarp;
-        const size_t smem = fixed + (size_t)ppc * slot_bytes;
-        // per-CTA partials: counts, sum, sum^2 per (lag, bin) and a Welford triple per lag
-        const size_t per_cta = (size_t)nl * a.n_bins * 24 + sizeof(WelfordPart) * (size_t)nl + 64;
-        const int64_t cap_grid = (int64_t)((kDmumuNoAllocBytes - 1024) / per_cta);
-        if (cap_grid < 1)
-            return fail(PT_ERR_ARG, "pt_dmumu_accumulate_device_noalloc: n_lags x n_bins too large for the " +
-                                        std::to_string(kDmumuNoAllocBytes >> 20) + " MiB fixed scratch");
-        void* kfn = small_idx ? (void*)dmumu_kernel<uint16_t, true, CacheSource>
-                              : (void*)dmumu_kernel<uint32_t, true, CacheSource>;
-        PT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        int per_sm = 1;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, threads, smem);
-        per_sm = std::max(1, per_sm);
-        const int64_t tiles = (a.n + ppc - 1) / ppc;
-        const int grid = (int)std::max<int64_t>(
-            1, std::min<int64_t>(std::min<int64_t>(tiles, (int64_t)ctx->num_sms * per_sm), cap_grid));
-        const size_t part_acc = (size_t)grid * nl * a.n_bins;
-        char* base = (char*)scratch;
-        DmumuLaunch L;
-        L.n = a.n; L.nsave = a.nsave;
-        L.start_cap = a.injection ? 1 : a.nsave;
-        L.lags = a.lags + lag0; L.nl = nl; L.edges = a.edges; L.n_bins = a.n_bins; L.bin_abs = a.bin_abs;
-        L.ppc = ppc; L.groups = groups; L.parts = parts; L.slot_bytes = slot_bytes;
-        L.part_cnt = (unsigned long long*)base;
-        L.part_sd = (double*)(base + align16(part_acc * 8));
-        L.part_sd2 = (double*)(base + 2 * align16(part_acc * 8));
-        L.part_w = (WelfordPart*)(base + 3 * align16(part_acc * 8));
-        L.gslots = nullptr;
-        if (3 * align16(part_acc * 8) + sizeof(WelfordPart) * (size_t)grid * nl > kDmumuNoAllocBytes)
-            return fail(PT_ERR_ARG, "internal: no-alloc scratch overflow");
-        if (small_idx) dmumu_kernel<uint16_t, true, CacheSource><<<grid, threads, smem, s>>>(L, src);
-        else dmumu_kernel<uint32_t, true, CacheSource><<<grid, threads, smem, s>>>(L, src);
-        PT_CHECK_LAUNCH("dmumu_kernel (no-alloc)");
-        const int fin_blocks = (int)((std::max(nl * a.n_bins, nl) + 255) / 256);
-        dmumu_finalize_kernel<<<fin_blocks, 256, 0, s>>>(L.part_cnt, L.part_sd, L.part_sd2, L.part_w, grid, nl,
-                                                         a.n_bins, lag0, a.n_lags, a.counts, a.sum_d, a.sum_d2,
-                                                         a.w_count, a.w_mean, a.w_m2, a.pair_ss, a.pair_n);
-        PT_CHECK_LAUNCH("dmumu_finalize_kernel (no-alloc)");
-    }
-    return PT_OK;
-}
-
-}  // namespace
-}  // namespace pt
-
-extern "C" int pt_dmumu_accumulate_device_noalloc(pt_ctx* ctx, const float* d_mu, int64_t n, int64_t nsave, int64_t sp,
-                                                  int64_t ss, const int64_t* d_lags, int n_lags, const double* d_edges,
-                                                  int n_bins, int start_mode, int bin_abs, int64_t* d_counts,
-                                                  double* d_sum_d, double* d_sum_d2, int64_t* d_w_count,
-                                                  double* d_w_mean, double* d_w_m2, double* d_pair_ss,
-                                                  int64_t* d_pair_n)
-{
-    using namespace pt;
-    if (!ctx) return fail(PT_ERR_ARG, "ctx is null");
-    if (n < 0 || nsave < 1 || n_lags < 0 || n_bins < 1) return fail(PT_ERR_ARG, "bad sizes");
-    if (start_mode != PT_START_SLIDING && start_mode != PT_START_INJECTION) return fail(PT_ERR_ARG, "start_mode");
-    if (n == 0 || n_lags == 0) return PT_OK;
-    if (!(d_mu && d_lags && d_edges && d_counts && d_sum_d && d_sum_d2 && d_w_count && d_w_mean && d_w_m2 &&
-          d_pair_ss && d_pair_n))
-        return fail(PT_ERR_ARG, "null pointer");
-    PT_DEVICE_SCOPE(ctx->device);
-    DmumuArgs a{d_mu, n, nsave, sp, ss, d_lags, n_lags, d_edges, n_bins, start_mode == PT_START_INJECTION, bin_abs != 0,
-                d_counts, d_sum_d, d_sum_d2, d_w_count, d_w_mean, d_w_m2, d_pair_ss, d_pair_n};
-    return run_dmumu_noalloc(ctx, a, ctx->stream);
-}

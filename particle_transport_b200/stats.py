@@ -264,7 +264,7 @@ def reconstruct_mu_chunk(positions, momenta, Bx, By, Bz, grid, dtype=np.float32)
 
 
 # --------------------------------------------------------------------------
-# limits of the D_mumu entry points (the launch arithmetic of lagstats.cu)
+# limits of the D_mumu entry points (dmumu_limits in dmumu.cu)
 # --------------------------------------------------------------------------
 _DMUMU_SMEM_BUDGET = 200 * 1024  # shared memory a D_mumu CTA may use (B200 opt-in maximum is 227 KiB)
 _DMUMU_NOALLOC_BYTES = 16 << 20  # the no-alloc entry's fixed device array

@@ -261,3 +261,55 @@ def test_phase_space_dmumu_fused_matches_oracle(cuda, oracle, dtype, mode, layou
     g = {k: v.cpu().numpy() for k, v in g.items()}
     check_dmumu(g, o)
     assert g["pair_counts"].sum() > 0
+
+
+def _nan_pattern(mu, pattern, rng):
+    """none; dead: NaN from some save on (open boundary); holes: NaN and Inf between finite saves; mixed."""
+    n, nsave = mu.shape
+    if pattern in ("dead", "mixed"):
+        at = rng.integers(0, nsave + 1, size=n)  # 0: never alive, nsave: never dead
+        sel = np.arange(n) % 2 == 0
+        mu[(np.arange(nsave)[None, :] >= at[:, None]) & sel[:, None]] = np.nan
+    if pattern in ("holes", "mixed"):
+        m = rng.random(mu.shape)
+        m[np.arange(n) % 3 == 0] = 1.0
+        mu[m < 0.03] = np.nan
+        mu[(m >= 0.03) & (m < 0.04)] = np.inf
+    return mu
+
+
+# the edges of the D_mumu launch shapes: one to eight lag sets of 8, then several lag groups and lag batches; one
+# particle to more than a round; series stored four times on chip, once on chip (12,000 saves), and in global memory
+# (30,000); injection tiles of 128 particles with a remainder, and lags beyond one warp
+@pytest.mark.parametrize("n,nsave,n_lags,n_bins,mode,layout,pattern", [
+    (1, 2, 1, 1, "sliding", "time_fastest", "none"),
+    (37, 33, 8, 4, "sliding", "particle_fastest", "dead"),
+    (700, 129, 9, 20, "sliding", "time_fastest", "mixed"),
+    (150, 4001, 64, 50, "sliding", "time_fastest", "dead"),
+    (301, 513, 41, 7, "sliding", "particle_fastest", "holes"),
+    (90, 700, 65, 24, "sliding", "time_fastest", "mixed"),
+    (64, 900, 130, 40, "sliding", "time_fastest", "dead"),
+    (20, 12000, 30, 16, "sliding", "time_fastest", "mixed"),
+    (5, 30000, 17, 40, "sliding", "particle_fastest", "mixed"),
+    (40, 260, 32, 290, "sliding", "time_fastest", "none"),
+    (1, 40, 5, 6, "injection", "time_fastest", "none"),
+    (129, 300, 33, 20, "injection", "particle_fastest", "mixed"),
+    (1000, 801, 64, 50, "injection", "time_fastest", "mixed"),
+    (5000, 97, 7, 10, "injection", "particle_fastest", "dead"),
+])
+def test_dmumu_shapes_and_nan_patterns(cuda, oracle, n, nsave, n_lags, n_bins, mode, layout, pattern):
+    """Counts bit for bit and sums to 1e-12 (as above) at the edges of the launch shapes, with lags past the series
+    and values outside the edges; the tolerance is the summation-order bound of the other cases."""
+    torch = cuda
+    rng = np.random.default_rng(n + nsave + n_lags)
+    mu = _nan_pattern(random_mu_cache(n, nsave, seed=nsave), pattern, rng)
+    lags = np.concatenate([log_spaced_lag_steps(nsave - 1, n_lags) if n_lags < nsave else np.arange(1, n_lags + 1),
+                           [nsave, 3 * nsave]])
+    rng.shuffle(lags)
+    edges = np.linspace(0.05, 0.9, n_bins + 1)
+    o = zero_dmumu(len(lags), n_bins)
+    oracle.dmumu_accumulate(mu, lags, edges, o, injection=mode == "injection", bin_abs=True)
+    d = torch.as_tensor(mu if layout == "time_fastest" else np.ascontiguousarray(mu.T), device="cuda")
+    acc = S.new_dmumu_accumulators(len(lags), n_bins, device="cuda")
+    gpu_dmumu(d, lags, edges, start_mode=mode, layout=layout, acc=acc)
+    check_dmumu({k: v.cpu().numpy() for k, v in acc.items()}, o)
