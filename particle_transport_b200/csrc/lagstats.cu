@@ -2,11 +2,10 @@
 //
 // D_pp (process_momenta_chunk_dpp_cpu!, src/compute_dpp_full.jl:247-288)
 // ---------------------------------------------------------------------
-// Same layout without bins: |p| is computed once per (particle, save) in FP64
-// and every lane keeps its lag's count, sum(dp) and sum(dp^2) in registers for
-// the whole launch; the normalised sums sum(dp/p0) = sum(dp)/p0 and
-// sum((dp/p0)^2) = sum(dp^2)/p0^2 are formed once per lag at the end, which
-// equals the reference's per-pair division up to rounding.
+// |p| is computed once per (particle, save) in FP64 and staged on chip; every
+// lag's count, sum(dp) and sum(dp^2) are added up there, and the normalised sums
+// sum(dp/p0) = sum(dp)/p0 and sum((dp/p0)^2) = sum(dp^2)/p0^2 are formed once per
+// lag at the end, which equals the reference's per-pair division up to rounding.
 #include <math_constants.h>
 
 #include "exact_mu.cuh"
@@ -38,136 +37,292 @@ struct DppPart {
     double sdp, sdp2;
 };
 
+constexpr int kDppThreads = 512;
+constexpr int kDppWarps = kDppThreads / kWarp;
+constexpr int kDppLags = 4;    // lags of a set: |p|[s] is read once for them
+constexpr int kDppUnroll = 2;  // starts per lane and pass
+
 struct DppLaunch {
-    const float* mom;
-    int64_t chunk, nsave;
+    const double* pmag;    // [n][pitch] |p| of this launch's particles
+    int64_t n, nsave, pitch;
     const int64_t* lags;
     int nl;
-    double p0;
-    int ppc, wps;  // particle slots per CTA, warps per slot
-    size_t slot_bytes;
-    char* gslots;
-    DppPart* part;  // [grid][nl]
+    int ppc;       // particle series per CTA
+    int sets;      // lag sets, a multiple of the warps
+    int first;     // 1: set the partials, 0: add to them
+    DppPart* part; // [grid][nl]
 };
 
-// Warps = (particle slot, lag subset): warp w of a slot owns lags w, w + wps,
-// w + 2 wps, ... and takes kDppLags of them at a time; its lanes take the
-// starts s = lane, lane + 32, ...  A warp's 8-byte |p| reads are then
-// consecutive (no shared-memory bank conflicts, whatever the lags), and
-// |p|[s] is read once for the lags of a pass.  The series of a slot holds |p| at saves 0..nsave-1 and
-// NaN at index nsave, so the end of a pair past the series reads NaN (an
-// invalid pair) with no bounds test.  A lag's sums are warp-reduced once per
-// particle and added by lane 0 into the slot's accumulator for that lag (one
-// writer per (slot, lag)); the CTA adds its slots in slot order at the end.
-// lags of a warp per pass over the starts (|p|[s] read once for them); 4 was
-// measured slower: a pass runs to the range of its smallest lag
-constexpr int kDppLags = 2;
-
-template <bool SMEM_SLOTS>
-__global__ void __launch_bounds__(1024) dpp_kernel(DppLaunch a)
+// |p| of particles [p0, p0 + n) at every save, time-fastest: out[p][s], pitch
+// doubles per particle.  A block turns kPmagSaves saves of 32 particles: rows of
+// 128 bytes in, rows of kPmagSaves doubles out.  A pass of its own because the pair
+// kernel holds three series per CTA: reading its particles there took a line per
+// save and component for 12 useful bytes, a fifth of that kernel's L1 wavefronts.
+// The launches alternate on particle chunks whose |p| stays in L2.
+constexpr int kPmagSaves = 32;
+__global__ void __launch_bounds__(256) pmag_kernel(const float* __restrict__ mom, int64_t chunk, int64_t nsave,
+                                                   int64_t p0, int64_t n, int64_t pitch, double* __restrict__ out)
 {
-    extern __shared__ __align__(16) unsigned char smem[];
-    // shared layout: acc[ppc][nl] | slots (when on chip)
-    DppPart* acc = (DppPart*)smem;
-    const size_t acc_bytes = ((size_t)a.ppc * a.nl * sizeof(DppPart) + 15) & ~(size_t)15;
-    unsigned char* slot_base =
-        SMEM_SLOTS ? smem + acc_bytes : (unsigned char*)(a.gslots + (size_t)blockIdx.x * a.ppc * a.slot_bytes);
-    for (int i = threadIdx.x; i < a.ppc * a.nl; i += blockDim.x) acc[i] = DppPart{0, 0.0, 0.0};
-    const int warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
-    const int slot = warp / a.wps, w = warp % a.wps;
-    const int nsave = (int)a.nsave;  // nsave < 2^31
-    double* series = (double*)(slot_base + (size_t)slot * a.slot_bytes);
-    const int64_t tiles = (a.chunk + a.ppc - 1) / a.ppc;
-    __syncthreads();
-    for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        // cooperative staging: thread t -> (save, particle slot)
-        const int64_t p0i = tile * a.ppc;
-        const int np = (int)(a.chunk - p0i < (int64_t)a.ppc ? a.chunk - p0i : (int64_t)a.ppc);
-        for (int64_t t = threadIdx.x; t < (int64_t)np * (a.nsave + 1); t += blockDim.x) {
-            const int sl = (int)(t % np);
-            const int64_t s = t / np;
-            double v = CUDART_NAN;  // the pad at index nsave
-            if (s < a.nsave) {
-                const float* m = a.mom + s * 3 * a.chunk + p0i + sl;
-                v = pmag_exact(m[0], m[a.chunk], m[2 * a.chunk]);
-            }
-            ((double*)(slot_base + (size_t)sl * a.slot_bytes))[s] = v;
+    __shared__ double tile[kWarp][kPmagSaves + 1];
+    const int x = threadIdx.x % kWarp, y = threadIdx.x / kWarp;
+    const int64_t s0 = (int64_t)blockIdx.x * kPmagSaves;
+    for (int64_t b = blockIdx.y; b * kWarp < n; b += gridDim.y) {
+        const int64_t q = b * kWarp + x;
+        float v[kPmagSaves / 8][3];
+#pragma unroll
+        for (int i = 0; i < kPmagSaves / 8; ++i) {
+            const int64_t s = s0 + y + 8 * i;
+            const float* m = mom + 3 * s * chunk + p0 + q;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) v[i][c] = s < nsave && q < n ? m[c * chunk] : 0.0f;
+        }
+#pragma unroll
+        for (int i = 0; i < kPmagSaves / 8; ++i) tile[x][y + 8 * i] = pmag_exact(v[i][0], v[i][1], v[i][2]);
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kWarp / 8; ++i) {
+            const int64_t r = b * kWarp + y + 8 * i;
+            if (r < n && s0 + x < nsave) out[r * pitch + s0 + x] = tile[y + 8 * i][x];
         }
         __syncthreads();
-        if (slot < np) {
-            // |p| >= 0 or NaN or +inf, so pe - ps is finite exactly when both
-            // ends are finite; an invalid pair adds 0 (branch-free), which
-            // leaves the sums unchanged.  The normalised sums are sum(d)/p0
-            // and sum(d^2)/p0^2, formed once per lag in dpp_finalize_kernel.
-            for (int l0 = w; l0 < a.nl; l0 += kDppLags * a.wps) {
-                int L[kDppLags], cnt[kDppLags];
-                double sd[kDppLags], sq[kDppLags];
-                int lmin = nsave;
-#pragma unroll
-                for (int k = 0; k < kDppLags; ++k) {
-                    const int l = l0 + k * a.wps;
-                    // the range test in 64 bits, before the narrowing
-                    const int64_t v64 = l < a.nl ? a.lags[l] : a.nsave;
-                    const int v = (v64 < 1 || v64 >= a.nsave) ? nsave : (int)v64;  // lag >= nsteps -> skipped
-                    L[k] = v;
-                    lmin = min(lmin, v);
-                    cnt[k] = 0;
-                    sd[k] = 0.0;
-                    sq[k] = 0.0;
-                }
-                const int lim = nsave - lmin;
-                for (int s = lane; s < lim; s += kWarp) {
-                    const double ps = series[s];
-#pragma unroll
-                    for (int k = 0; k < kDppLags; ++k) {
-                        const double pe = series[min((unsigned)s + (unsigned)L[k], (unsigned)nsave)];
-                        double d = pe - ps;
-                        const bool ok = isfinite(d);
-                        d = ok ? d : 0.0;
-                        cnt[k] += (int)ok;
-                        sd[k] += d;
-                        sq[k] = fma(d, d, sq[k]);
-                    }
-                }
-#pragma unroll
-                for (int k = 0; k < kDppLags; ++k) {
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) {
-                        cnt[k] += __shfl_xor_sync(0xffffffffu, cnt[k], o);
-                        sd[k] += __shfl_xor_sync(0xffffffffu, sd[k], o);
-                        sq[k] += __shfl_xor_sync(0xffffffffu, sq[k], o);
-                    }
-                    const int l = l0 + k * a.wps;
-                    if (lane == 0 && l < a.nl) {
-                        DppPart& A = acc[slot * a.nl + l];
-                        A.count += cnt[k]; A.sdp += sd[k]; A.sdp2 += sq[k];
-                    }
-                }
-            }
-        }
-        __syncthreads();
-    }
-    // CTA epilogue: slots added in slot order
-    for (int l = threadIdx.x; l < a.nl; l += blockDim.x) {
-        DppPart r{0, 0, 0};
-        for (int sl = 0; sl < a.ppc; ++sl) {
-            const DppPart v = acc[sl * a.nl + l];
-            r.count += v.count; r.sdp += v.sdp; r.sdp2 += v.sdp2;
-        }
-        a.part[(int64_t)blockIdx.x * a.nl + l] = r;
     }
 }
 
-__global__ void dpp_finalize_kernel(const DppPart* __restrict__ part, int grid, int nl, int lag0, double p0,
-                                    int64_t* counts, double* sdp, double* sdp2, double* sdn, double* sdn2)
+struct DppFixed {
+    size_t sd2, cnt, sorted, idx, nfin, fin, series;
+};
+__host__ __device__ inline DppFixed dpp_fixed(int sets, int nl, int ppc)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nl) return;
+    auto a16 = [](size_t v) { return (v + 15) & ~(size_t)15; };
+    DppFixed f;
+    f.sd2 = (size_t)sets * kDppLags * sizeof(double);
+    f.cnt = 2 * f.sd2;
+    f.sorted = f.cnt + sizeof(unsigned long long) * nl;
+    f.idx = f.sorted + sizeof(int) * nl;
+    f.nfin = f.idx + sizeof(int) * nl;
+    f.fin = f.nfin + sizeof(int) * ppc;
+    f.series = a16(f.fin + sizeof(int) * ppc);
+    return f;
+}
+
+// Starts [s0, s1) against NL lags: p[s + L[k]] - p[s], added to sd[k] and sq[k].
+// TEST: only finite differences count (into cnt).
+template <int NL, bool TEST>
+__device__ __forceinline__ void dpp_rows(const double* __restrict__ p, int s0, int s1, const int (&L)[kDppLags], int lane,
+                                         double (&sd)[kDppLags], double (&sq)[kDppLags], int (&cnt)[kDppLags])
+{
+    auto pair = [&](double ps, double pe, int k) {
+        double d = pe - ps;
+        if constexpr (TEST) {
+            const bool ok = isfinite(d);
+            d = ok ? d : 0.0;
+            cnt[k] += (int)ok;
+        }
+        sd[k] += d;
+        sq[k] = fma(d, d, sq[k]);
+    };
+    int s = s0 + lane;
+    for (; s + (kDppUnroll - 1) * kWarp < s1; s += kDppUnroll * kWarp) {
+        double ps[kDppUnroll], pe[kDppUnroll][NL];
+#pragma unroll
+        for (int u = 0; u < kDppUnroll; ++u) {
+            ps[u] = p[s + u * kWarp];
+#pragma unroll
+            for (int k = 0; k < NL; ++k) pe[u][k] = p[s + L[k] + u * kWarp];
+        }
+#pragma unroll
+        for (int u = 0; u < kDppUnroll; ++u)
+#pragma unroll
+            for (int k = 0; k < NL; ++k) pair(ps[u], pe[u][k], k);
+    }
+    for (; s < s1; s += kWarp) {
+        const double ps = p[s];
+#pragma unroll
+        for (int k = 0; k < NL; ++k) pair(ps, p[s + L[k]], k);
+    }
+}
+
+// Lags are dealt to sets of at most kDppLags, in the order of their value back and
+// forth over the sets, so that the sets have about equal numbers of pairs; a warp
+// owns a set (or every 16th) for all particles, its lanes take consecutive starts,
+// and the lanes' sums are added across the warp once per tile of particles.  A
+// warp's 8-byte |p| reads are consecutive (no bank conflicts, whatever the lags),
+// and |p|[s] is read once for the set's lags.
+//
+// A particle whose finite saves are a prefix [0, nfin) needs no test in the pair
+// loop: the starts below nfin - L are exactly lag L's pairs, so a set runs its
+// lags together up to the longest one's end, the others on to the next one's, and
+// so on, and the count of a lag is max(0, nfin - L).  Other particles take the same
+// loops up to nsave - L with a finite test per pair.
+//
+// A set's sums have one writer and CTAs are added in order: the result is
+// deterministic.
+//
+// Bound by shared-memory bandwidth: 8 bytes per pair and 8 per start and set,
+// about 2.6 cycles of the SM's 128 B/clk per 32 pairs, with the FP64 pipe at 1.5.
+// Two CTAs per SM, so that one's staging runs under the other's pairs.
+// 65,536 x 4001 saves x 55 lags with 16 energy snapshots and histograms: 8.45 ms
+// with two lags per pass, a finite test per pair and the reads of the momenta in
+// this kernel; 5.75 ms now (4.85 ms here, 0.85 ms in pmag_kernel).
+template <bool SMEM_SLOTS>
+__global__ void __launch_bounds__(kDppThreads, 2) dpp_kernel(DppLaunch a)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int nl = a.nl, nsave = (int)a.nsave, ppc = a.ppc, sets = a.sets;
+    const DppFixed F = dpp_fixed(sets, nl, ppc);
+    double* acc_sd = (double*)smem;  // [set][kDppLags]
+    double* acc_sd2 = (double*)(smem + F.sd2);
+    unsigned long long* acc_cnt = (unsigned long long*)(smem + F.cnt);  // [lag, by value]
+    int* s_lag = (int*)(smem + F.sorted);  // ascending; nsave where no pair exists
+    int* s_idx = (int*)(smem + F.idx);     // index of the lag in a.lags
+    int* s_nfin = (int*)(smem + F.nfin);   // first non-finite save
+    int* s_fin = (int*)(smem + F.fin);     // finite saves
+    double* series = (double*)(smem + F.series);  // [ppc][pitch]
+    for (int i = threadIdx.x; i < sets * kDppLags; i += blockDim.x) acc_sd[i] = acc_sd2[i] = 0.0;
+    for (int i = threadIdx.x; i < nl; i += blockDim.x) {
+        acc_cnt[i] = 0ull;
+        auto value = [&](int q) {  // the range test in 64 bits, before the narrowing
+            const int64_t v = a.lags[q];
+            return v < 1 || v >= a.nsave ? nsave : (int)v;  // lag >= nsteps -> skipped
+        };
+        const int L = value(i);
+        int rank = 0;
+        for (int q = 0; q < nl; ++q) {
+            const int Lq = value(q);
+            rank += Lq < L || (Lq == L && q < i);
+        }
+        s_lag[rank] = L;
+        s_idx[rank] = i;
+    }
+    __syncthreads();  // a CTA without a tile goes straight to the partials
+    const int warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
+    // lag k of a set, by value: rows of `sets` lags dealt forth and back
+    auto dealt = [&](int set, int k) { return k * sets + (k & 1 ? sets - 1 - set : set); };
+    const int64_t tiles = (a.n + ppc - 1) / ppc;
+    for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int64_t p0 = tile * ppc;
+        const int np = (int)min(a.n - p0, (int64_t)ppc);
+        const double* from = a.pmag + p0 * a.pitch;
+        for (int i = threadIdx.x; i < ppc; i += blockDim.x) {
+            s_nfin[i] = nsave;
+            s_fin[i] = 0;
+        }
+        __syncthreads();
+        for (int q = 0; q < np; ++q) {
+            int bad = nsave, fin = 0;
+            auto look = [&](double v, int s) {
+                if (s >= nsave) return;
+                if (isfinite(v)) ++fin;
+                else bad = min(bad, s);
+            };
+            // two saves at a time: the pitch is even and the rows 16-byte aligned
+            const double2* row = (const double2*)(from + q * a.pitch);
+#pragma unroll 4
+            for (int i = threadIdx.x; i < (int)(a.pitch / 2); i += blockDim.x) {
+                const double2 v = row[i];
+                if (SMEM_SLOTS) ((double2*)(series + q * a.pitch))[i] = v;
+                look(v.x, 2 * i);
+                look(v.y, 2 * i + 1);
+            }
+            if (bad < nsave) atomicMin(&s_nfin[q], bad);
+#pragma unroll
+            for (int o = kWarp / 2; o > 0; o >>= 1) fin += __shfl_xor_sync(0xffffffffu, fin, o);
+            if (lane == 0) atomicAdd(&s_fin[q], fin);
+        }
+        __syncthreads();
+        for (int l = threadIdx.x; l < nl; l += blockDim.x) {
+            long long c = 0;
+            for (int q = 0; q < np; ++q)
+                if (s_fin[q] == s_nfin[q]) c += max(0, s_nfin[q] - s_lag[l]);
+            if (c > 0) atomicAdd(&acc_cnt[l], (unsigned long long)c);
+        }
+        for (int set = warp; set < sets; set += kDppWarps) {
+            int L[kDppLags], cnt[kDppLags];
+            double sd[kDppLags], sq[kDppLags];
+#pragma unroll
+            for (int k = 0; k < kDppLags; ++k) {
+                const int l = dealt(set, k);
+                L[k] = l < nl ? s_lag[l] : nsave;
+                cnt[k] = 0;
+                sd[k] = sq[k] = 0.0;
+            }
+            for (int q = 0; q < np; ++q) {
+                const bool prefix = s_fin[q] == s_nfin[q];
+                const int end = prefix ? s_nfin[q] : nsave;
+                int lim[kDppLags];  // falls with k
+#pragma unroll
+                for (int k = 0; k < kDppLags; ++k) lim[k] = max(0, end - L[k]);
+                const double* p = (SMEM_SLOTS ? (const double*)series : from) + q * a.pitch;
+                if (prefix) {
+                    dpp_rows<4, false>(p, 0, lim[3], L, lane, sd, sq, cnt);
+                    dpp_rows<3, false>(p, lim[3], lim[2], L, lane, sd, sq, cnt);
+                    dpp_rows<2, false>(p, lim[2], lim[1], L, lane, sd, sq, cnt);
+                    dpp_rows<1, false>(p, lim[1], lim[0], L, lane, sd, sq, cnt);
+                } else {
+                    dpp_rows<4, true>(p, 0, lim[3], L, lane, sd, sq, cnt);
+                    dpp_rows<3, true>(p, lim[3], lim[2], L, lane, sd, sq, cnt);
+                    dpp_rows<2, true>(p, lim[2], lim[1], L, lane, sd, sq, cnt);
+                    dpp_rows<1, true>(p, lim[1], lim[0], L, lane, sd, sq, cnt);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < kDppLags; ++k) {
+#pragma unroll
+                for (int o = kWarp / 2; o > 0; o >>= 1) {
+                    sd[k] += __shfl_xor_sync(0xffffffffu, sd[k], o);
+                    sq[k] += __shfl_xor_sync(0xffffffffu, sq[k], o);
+                    cnt[k] += __shfl_xor_sync(0xffffffffu, cnt[k], o);
+                }
+                if (lane == 0) {
+                    acc_sd[set * kDppLags + k] += sd[k];
+                    acc_sd2[set * kDppLags + k] += sq[k];
+                    const int l = dealt(set, k);
+                    if (l < nl && cnt[k] > 0) atomicAdd(&acc_cnt[l], (unsigned long long)cnt[k]);
+                }
+            }
+        }
+        __syncthreads();
+    }
+    for (int i = threadIdx.x; i < sets * kDppLags; i += blockDim.x) {
+        const int l = dealt(i / kDppLags, i % kDppLags);
+        if (l >= nl) continue;
+        DppPart& out = a.part[(int64_t)blockIdx.x * nl + s_idx[l]];
+        DppPart r{(long long)acc_cnt[l], acc_sd[i], acc_sd2[i]};
+        if (!a.first) {
+            r.count += out.count;
+            r.sdp += out.sdp;
+            r.sdp2 += out.sdp2;
+        }
+        out = r;
+    }
+}
+
+// One block per lag: threads add the CTAs t, t + 256, ... and a tree adds the
+// threads, a fixed order.  (One thread per lag walking all CTAs took 48 us.)
+constexpr int kDppFinThreads = 256;
+__global__ void __launch_bounds__(kDppFinThreads)
+    dpp_finalize_kernel(const DppPart* __restrict__ part, int grid, int nl, int lag0, double p0, int64_t* counts,
+                        double* sdp, double* sdp2, double* sdn, double* sdn2)
+{
+    __shared__ DppPart sh[kDppFinThreads];
+    const int t = blockIdx.x;
     DppPart r{0, 0, 0};
-    for (int g = 0; g < grid; ++g) {
+    for (int g = threadIdx.x; g < grid; g += kDppFinThreads) {
         const DppPart q = part[(int64_t)g * nl + t];
         r.count += q.count; r.sdp += q.sdp; r.sdp2 += q.sdp2;
     }
+    sh[threadIdx.x] = r;
+    __syncthreads();
+    for (int w = kDppFinThreads / 2; w > 0; w >>= 1) {
+        if ((int)threadIdx.x < w) {
+            const DppPart q = sh[threadIdx.x + w];
+            DppPart& m = sh[threadIdx.x];
+            m.count += q.count; m.sdp += q.sdp; m.sdp2 += q.sdp2;
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x != 0) return;
+    r = sh[0];
     const int l = lag0 + t;
     counts[l] += r.count;
     sdp[l] += r.sdp;
@@ -364,56 +519,60 @@ int run_dmumu_phase_space(pt_ctx* ctx, const DmumuArgs& a, const void* pos, cons
 int run_dpp(pt_ctx* ctx, const DppArgs& a, cudaStream_t s)
 {
     if (a.chunk <= 0 || a.n_lags <= 0) return PT_OK;
-    int max_smem = 0;
-    cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
-    const size_t budget = (size_t)std::min(max_smem, 200 * 1024);
     if (a.nsave >= INT32_MAX) return fail(PT_ERR_ARG, "nsave must be below 2^31");
-    const size_t slot_bytes = align16(sizeof(double) * (size_t)(a.nsave + 1));  // + NaN pad
+    int max_smem = 0, sm_smem = 0;
+    cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
+    cudaDeviceGetAttribute(&sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx->device);
+    const int64_t pitch = (a.nsave + 1) & ~(int64_t)1;
+    const size_t series = sizeof(double) * (size_t)pitch;
     const int nl_cap = 32 * 8;
     for (int lag0 = 0; lag0 < a.n_lags; lag0 += nl_cap) {
         const int nl = std::min(nl_cap, a.n_lags - lag0);
-        // particle slots per CTA (series on chip when they fit) and warps per
-        // slot (each takes ceil(nl / wps) lags, two at a time)
-        const size_t acc_per_slot = sizeof(DppPart) * (size_t)nl;
-        bool smem_slots = align16(acc_per_slot) + slot_bytes <= budget;
-        // the most warps per CTA (at most 32), the larger ppc among equals:
-        // at 55 lags and room for five series, 4 slots x 8 warps measured
-        // 1.45e12 lag-pairs/s against 1.32e12 for 5 x 6
-        const int max_ppc = smem_slots ? (int)std::min<size_t>(budget / (slot_bytes + acc_per_slot), 8) : 4;
-        const int lag_sets = (nl + kDppLags - 1) / kDppLags;
-        int ppc = 1, wps = 1, best = 0;
-        for (int c = 1; c <= std::max(1, max_ppc); ++c) {
-            const int w = std::max(1, std::min(32 / c, lag_sets));
-            if (c * w >= best) {
-                best = c * w;
-                ppc = c;
-                wps = w;
-            }
-        }
-        const int threads = ppc * wps * kWarp;
-        const size_t smem = align16(acc_per_slot * ppc) + (smem_slots ? (size_t)ppc * slot_bytes : 0);
-        const int64_t tiles = (a.chunk + ppc - 1) / ppc;
+        DppLaunch L;
+        L.sets = kDppWarps * ((nl + kDppWarps * kDppLags - 1) / (kDppWarps * kDppLags));
+        // Series on chip when they fit, two CTAs per SM when half of it holds one
+        // (the reserved KB per CTA left out).  As many as fit, up to 16, but no
+        // more than gives every CTA of the chip a tile.
+        const size_t half = std::min<size_t>(max_smem, sm_smem / 2 - 1024);
+        auto need = [&](int ppc) { return dpp_fixed(L.sets, nl, ppc).series + (size_t)ppc * series; };
+        const bool two = need(1) <= half;
+        const bool smem_slots = two || need(1) <= (size_t)max_smem;
+        int ppc = 1;
+        while (smem_slots && ppc < 16 && (int64_t)ppc * ctx->num_sms * (two ? 2 : 1) < a.chunk &&
+               need(ppc + 1) <= (two ? half : (size_t)max_smem))
+            ++ppc;
+        const size_t smem = smem_slots ? need(ppc) : dpp_fixed(L.sets, nl, ppc).series;
         void* kfn = smem_slots ? (void*)dpp_kernel<true> : (void*)dpp_kernel<false>;
         PT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         int per_sm = 1;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, threads, smem);
-        per_sm = std::max(1, per_sm);
-        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)ctx->num_sms * per_sm));
-        const size_t bytes = align16(sizeof(DppPart) * (size_t)grid * nl) +
-                             (smem_slots ? 0 : (size_t)grid * ppc * slot_bytes);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, kDppThreads, smem);
+        const int64_t ctas = (int64_t)ctx->num_sms * std::max(1, per_sm);
+        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((a.chunk + ppc - 1) / ppc, ctas));
+        // |p| chunks: whole rounds of the CTAs, as many as 128 MB hold
+        const int64_t round = (int64_t)grid * ppc;
+        const int64_t rounds = std::max<int64_t>(1, (int64_t)(((size_t)128 << 20) / series) / round);
+        const int64_t step = std::min<int64_t>(a.chunk, round * rounds);
+        const size_t part_bytes = (sizeof(DppPart) * (size_t)grid * nl + 255) & ~(size_t)255;
         void* scratch = nullptr;
-        int rc = scratch_get(ctx, 1, bytes, &scratch);
+        int rc = scratch_get(ctx, 1, part_bytes + (size_t)step * series, &scratch);
         if (rc) return rc;
-        DppLaunch L;
-        L.mom = a.mom; L.chunk = a.chunk; L.nsave = a.nsave; L.lags = a.lags + lag0; L.nl = nl; L.p0 = a.p0;
-        L.ppc = ppc; L.wps = wps; L.slot_bytes = slot_bytes;
+        double* pmag = (double*)((char*)scratch + part_bytes);
+        L.pmag = pmag; L.nsave = a.nsave; L.pitch = pitch; L.lags = a.lags + lag0; L.nl = nl;
+        L.ppc = ppc;
         L.part = (DppPart*)scratch;
-        L.gslots = smem_slots ? nullptr : (char*)scratch + align16(sizeof(DppPart) * (size_t)grid * nl);
-        if (smem_slots) dpp_kernel<true><<<grid, threads, smem, s>>>(L);
-        else dpp_kernel<false><<<grid, threads, smem, s>>>(L);
-        PT_CHECK_LAUNCH("dpp_kernel");
-        dpp_finalize_kernel<<<(nl + 255) / 256, 256, 0, s>>>(L.part, grid, nl, lag0, a.p0, a.counts, a.sdp, a.sdp2,
-                                                             a.sdn, a.sdn2);
+        for (int64_t p0 = 0; p0 < a.chunk; p0 += step) {
+            L.n = std::min(step, a.chunk - p0);
+            L.first = p0 == 0;
+            const dim3 pg((unsigned)((a.nsave + kPmagSaves - 1) / kPmagSaves),
+                          (unsigned)std::min<int64_t>((L.n + kWarp - 1) / kWarp, 65535));
+            pmag_kernel<<<pg, 256, 0, s>>>(a.mom, a.chunk, a.nsave, p0, L.n, pitch, pmag);
+            PT_CHECK_LAUNCH("pmag_kernel");
+            if (smem_slots) dpp_kernel<true><<<grid, kDppThreads, smem, s>>>(L);
+            else dpp_kernel<false><<<grid, kDppThreads, smem, s>>>(L);
+            PT_CHECK_LAUNCH("dpp_kernel");
+        }
+        dpp_finalize_kernel<<<nl, kDppFinThreads, 0, s>>>(L.part, grid, nl, lag0, a.p0, a.counts, a.sdp, a.sdp2,
+                                                          a.sdn, a.sdn2);
         PT_CHECK_LAUNCH("dpp_finalize_kernel");
     }
     return PT_OK;

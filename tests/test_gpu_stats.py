@@ -313,3 +313,38 @@ def test_dmumu_shapes_and_nan_patterns(cuda, oracle, n, nsave, n_lags, n_bins, m
     acc = S.new_dmumu_accumulators(len(lags), n_bins, device="cuda")
     gpu_dmumu(d, lags, edges, start_mode=mode, layout=layout, acc=acc)
     check_dmumu({k: v.cpu().numpy() for k, v in acc.items()}, o)
+
+
+# the edges of the D_pp launch shapes: one lag to more than 16 sets of 4, series counts of a CTA with a remainder, a
+# last |p| chunk with fewer tiles than CTAs (2400 x 6000 saves), one series per CTA (13,000 saves), one CTA per SM
+# (20,000), series in global memory (30,000)
+@pytest.mark.parametrize("chunk,nsave,n_lags,pattern", [
+    (1, 2, 1, "none"), (33, 65, 3, "dead"), (1000, 257, 16, "mixed"), (7, 300, 17, "holes"), (501, 402, 65, "dead"),
+    (2400, 6000, 12, "mixed"), (40, 13000, 20, "dead"), (9, 20000, 9, "mixed"), (3, 30000, 66, "dead"),
+])
+def test_dpp_shapes_and_nan_patterns(cuda, oracle, chunk, nsave, n_lags, pattern):
+    """As test_dpp_matches_oracle (counts exact, sums to 1e-12 of the sums the rounding acts on), on the device entry,
+    with particles that die and NaN or Inf between finite saves, and lags past the series."""
+    torch = cuda
+    rng = np.random.default_rng(chunk + nsave)
+    p = 5.4e-19 * (1 + 1e-3 * np.cumsum(rng.normal(size=(nsave, 1, chunk)), axis=0))
+    u = rng.normal(size=(nsave, 3, chunk))
+    u /= np.linalg.norm(u, axis=1, keepdims=True)
+    mom = (p * u).astype(np.float32)
+    hide = _nan_pattern(np.zeros((chunk, nsave), np.float32), pattern, rng).T
+    mom[:, 1] = np.where(np.isfinite(hide), mom[:, 1], hide)
+    mom = np.ascontiguousarray(mom)
+    lags = np.concatenate([log_spaced_lag_steps(nsave - 1, n_lags), [nsave, 2 * nsave]])
+    rng.shuffle(lags)
+    p0 = 5.4e-19
+    o = zero_dpp(len(lags))
+    oracle.dpp_accumulate(mom, lags, p0, o)
+    acc = S.new_dpp_accumulators(len(lags), device="cuda")
+    S.process_momenta_chunk_dpp(torch.as_tensor(mom, device="cuda"), lags, p0, acc["counts"], acc["sum_delta_p"],
+                                acc["sum_delta_p2"], acc["sum_delta_p_norm"], acc["sum_delta_p_norm2"])
+    g = {k: v.cpu().numpy() for k, v in acc.items()}
+    assert np.array_equal(g["counts"], o["counts"])
+    assert close(g["sum_delta_p2"], o["sum_dp2"])
+    assert close(g["sum_delta_p_norm2"], o["sum_dpn2"])
+    assert close(g["sum_delta_p"], o["sum_dp"], scale=np.sqrt(np.maximum(o["counts"], 1) * o["sum_dp2"]))
+    assert close(g["sum_delta_p_norm"], o["sum_dpn"], scale=np.sqrt(np.maximum(o["counts"], 1) * o["sum_dpn2"]))
