@@ -91,7 +91,8 @@ typedef struct {
     int32_t steps_per_launch; /* steps kept in registers per launch; 0 = auto           */
     int32_t sort_every;       /* F32 form: re-sort particles by brick every N steps; 0 off */
     int32_t kernel_variant;   /* F32 form: launch shape, threads per block x resident
-                                 blocks per SM: 0 = auto (= 1), 1 = 256 x occupancy,
+                                 blocks per SM: 0 = auto (one block, sized by the storage
+                                 and the particle count), 1 = 256 x occupancy,
                                  2 = 256 x 4, 3 = 128 x 8, 4 = 512 x 2, 5 = 256 x 1,
                                  6 = 512 x 1, 7 = 128 x 3, 8 = 128 x 2; BRICK_BF16
                                  fields: 9 = as 1 with half of the corners fetched

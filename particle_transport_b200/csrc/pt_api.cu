@@ -93,8 +93,8 @@ uint32_t spread3(uint32_t v)
 // Node offsets of the Morton-bricked layout: node(i, j, k) = offx[i] + offy[j] + offz[k].
 // Inside an 8^3 brick nodes are in Morton order (a 2x2x2 cell corner set is
 // 8 consecutive nodes when the cell is even-aligned); bricks are in Morton
-// order when the brick grid is a power-of-two cube, else x-fastest.
-void brick_offsets(const pt_grid& g, std::vector<uint32_t>& offs, int64_t& n_nodes)
+// order when the brick grid is a power-of-two cube (returned), else x-fastest.
+bool brick_offsets(const pt_grid& g, std::vector<uint32_t>& offs, int64_t& n_nodes)
 {
     const int64_t nbx = (g.nx + 7) / 8, nby = (g.ny + 7) / 8, nbz = (g.nz + 7) / 8;
     const bool cube_pow2 = nbx == nby && nby == nbz && (nbx & (nbx - 1)) == 0 && nbx <= 128;
@@ -108,6 +108,7 @@ void brick_offsets(const pt_grid& g, std::vector<uint32_t>& offs, int64_t& n_nod
         offs[g.nx + g.ny + k] = cube_pow2 ? (spread3((uint32_t)k) << 2)
                                           : (uint32_t)((k >> 3) * 512 * nbx * nby + (spread3((uint32_t)(k & 7)) << 2));
     n_nodes = cube_pow2 ? (8 * nbx) * (8 * nbx) * (8 * nbx) : 512 * nbx * nby * nbz;
+    return cube_pow2;
 }
 
 int field_create(pt_ctx* ctx, const double* const comps[6], bool on_device, const pt_grid* grid, int storage,
@@ -163,7 +164,7 @@ int field_create(pt_ctx* ctx, const double* const comps[6], bool on_device, cons
         return PT_OK;
     }
     std::vector<uint32_t> offs;
-    brick_offsets(*grid, offs, f->n_nodes);
+    f->morton = brick_offsets(*grid, offs, f->n_nodes);
     const size_t node_bytes = record_bytes(storage);
     cudaError_t e = cudaMalloc(&f->nodes, node_bytes * (size_t)f->n_nodes);
     if (e == cudaSuccess) e = cudaMalloc((void**)&f->offs, sizeof(uint32_t) * offs.size());
@@ -248,6 +249,7 @@ PushArgsFast fast_args(const pt_field* f, pt_fast_state* st, const pt_push_param
     a.fld.nx = g.nx; a.fld.ny = g.ny; a.fld.nz = g.nz;
     a.fld.bf16 = f->storage != PT_FIELD_BRICK_F32;
     a.fld.layout = field_layout(f->storage);
+    a.fld.morton = f->morton;
     a.fld.tex = f->tex;
     for (int c = 0; c < 3; ++c) a.fld.boff[c] = f->boff[c];
     a.wx = (g.xmax - g.xmin) / g.dx;
@@ -286,6 +288,7 @@ static int advance_exact_brick(pt_ctx* ctx, const pt_field* f, double* d_x1, dou
     a.nodes = f->nodes;
     a.tail = (const char*)f->nodes + 32 * (size_t)f->n_nodes;
     a.offs = f->offs;
+    a.morton = f->morton;
     a.g = f->grid;
     a.n = n; a.dt = p->dt; a.nsteps = p->nsteps; a.stride = p->stride;
     a.periodic = p->periodic; a.cache_mode = p->cache_mode; a.cache_f64 = p->cache_f64;

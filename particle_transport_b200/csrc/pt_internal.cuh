@@ -98,6 +98,7 @@ struct pt_field {
     void* nodes = nullptr;
     int64_t n_nodes = 0;
     uint32_t* offs = nullptr;  // [nx + ny + nz]: offx, offy, offz
+    bool morton = false;       // offs are Morton offsets (power-of-two cube)
     int64_t bytes = 0;
     cudaTextureObject_t tex = 0;  // brick forms: node records as uint4 texels (0 if over the texture limit)
     // BF16 forms: the mean of B / B_ref per component, subtracted before the
@@ -152,6 +153,20 @@ int staged_d2h(const std::vector<HostSeg>& segs, char* stage, size_t chunk, int 
 int64_t count_nonzero(const uint8_t* v, int64_t n);
 
 // ---------------------------------------------------------------- launches
+// Threads per block of a push with one block per SM, at most `most` (a multiple
+// of 128): the fewest that take n particles in as many passes over the chip, in
+// whole warps up to 128 and multiples of 128 (a warp per scheduler) beyond.
+inline int spread_threads(int64_t n, int most)
+{
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int64_t per_pass = (int64_t)sms * most, passes = std::max<int64_t>(1, (n + per_pass - 1) / per_pass);
+    const int64_t t = std::max<int64_t>(1, (n + sms * passes - 1) / (sms * passes));
+    const int64_t unit = t <= 128 ? 32 : 128;
+    return (int)std::min<int64_t>(most, (t + unit - 1) / unit * unit);
+}
+
 struct PushArgsRef {
     const double* f[6];
     pt_grid g;
@@ -177,6 +192,7 @@ struct PushArgsExactBrick {
     const void* nodes;     // head plane: (Bx, By, Bz, ux) per node, 32 bytes
     const void* tail;      // tail plane: (uy, uz) per node, 16 bytes
     const uint32_t* offs;  // [nx + ny + nz] per-axis node offsets
+    int morton;            // 1: they are the Morton offsets of a power-of-two cube
     pt_grid g;
     double* x[3];
     double* p[3];
@@ -223,12 +239,27 @@ inline bool fast_storage(int storage)
     return storage == PT_FIELD_BRICK_F32 || storage == PT_FIELD_BRICK_BF16 || storage == PT_FIELD_BRICK_BF16_XPAIR;
 }
 
+// Node offsets of power-of-two cubes, whose nodes and bricks are both in Morton
+// order (pt_field.morton): offx = morton10, offy = 2 morton10, offz = 4 morton10.
+// every third bit, and the bits of v < 1024 spread to them
+constexpr uint32_t kMorton = 0x09249249u;
+__device__ __forceinline__ uint32_t morton10(uint32_t v)
+{
+    v = (v * 0x00010001u) & 0xff0000ffu;
+    v = (v * 0x00000101u) & 0x0f00f00fu;
+    v = (v * 0x00000011u) & 0xc30c30c3u;
+    return (v * 0x00000005u) & 0x49249249u;
+}
+// morton10(v + 1) of morton10(v): the carry runs through the filled gaps
+__device__ __forceinline__ uint32_t morton_next(uint32_t m) { return ((m | ~kMorton) + 1u) & kMorton; }
+
 struct FieldArgsBrick {
     const void* nodes;
     const uint32_t* offs;
     int64_t nx, ny, nz;
     int bf16;    // 1 for the BF16 forms
     int layout;  // LAYOUT_*
+    int morton;  // 1: offs are the Morton offsets of a power-of-two cube
     cudaTextureObject_t tex;  // the node records as a linear uint4 texture (0: none)
     float boff[3];            // BF16 forms: mean field added back after the interpolation
 };

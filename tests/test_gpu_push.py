@@ -335,3 +335,29 @@ def test_time_fastest_rejected_where_it_does_not_apply(cuda):
     with pytest.raises(PtError, match="cache_pitch must be 0"):
         R.run_push_host(fb, copy_state(pb.state), np.ones(64, np.uint8),
                         R.push_params(pb.dt, 21, 4, cache="mu", precision="f32", cache_pitch=8), lambda i, r: None)
+
+
+# particle counts at the edges of the auto launch shape: one particle, a warp and one more, just over a warp per SM
+# times four, over one pass of 640 threads per SM; node offsets computed (16^3, Morton) and read from tables (20^3)
+@pytest.mark.parametrize("grid", [16, 20])
+@pytest.mark.parametrize("storage", ["brick_f32", "brick_bf16", "brick_bf16x"])
+@pytest.mark.parametrize("n", [1, 33, 148 * 128 + 1, 148 * 640 + 5])
+def test_auto_shape_bit_identical(cuda, storage, grid, n):
+    """The auto launch shape gives the trajectories of the fixed one, bit for bit."""
+    pb = small_problem(n=grid, n_particles=n, u_over_c=1e-4, energy_GeV=3.0)
+    mu_a, st_a, _ = _fast_mu(pb, storage, 24, 4, sort_every=8, variant=0)
+    mu_b, st_b, _ = _fast_mu(pb, storage, 24, 4, sort_every=8, variant=1)
+    assert np.array_equal(mu_a, mu_b, equal_nan=True)
+    for k in R.KEYS:
+        assert np.array_equal(st_a[k], st_b[k]), k
+
+
+@pytest.mark.parametrize("n", [5, 148 * 32 + 1, 148 * 256 + 1])
+@pytest.mark.parametrize("storage", ["ref_f64", "brick_f64"])
+def test_fp64_push_particle_counts(cuda, storage, n):
+    """The FP64 push at the edges of its launch shape (particles spread over all SMs) against the oracle."""
+    pb = small_problem(n=16, n_particles=n, u_over_c=1e-4, energy_GeV=3.0)
+    (mu_o, _, st_o, _), (col, _, st_g, _) = run_both(pb, 13, 3, "mu", storage=storage)
+    assert np.array_equal(mu_o, col.mu, equal_nan=True)
+    for k in R.KEYS:
+        assert np.array_equal(st_o[k], st_g[k]), k
