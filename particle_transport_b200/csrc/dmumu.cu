@@ -744,7 +744,7 @@ constexpr int kInjThreads = 512;
 struct DmumuInjection {
     const void* mu;            // element (p, s) at mu[p * sp + s * ss]
     int64_t sp, ss;
-    int packed;                // 1: save 0 and the batch's lags are the series' saves 0, first, first + 1, ...
+    int packed;                // 1: the series holds save 0 and then lag saves, this batch's from `first` on
     int first;
     int64_t n, nsave;
     const int64_t* lags;
@@ -1042,7 +1042,8 @@ int finalize(const DmumuArgs& a, const unsigned long long* cnt, const double* sd
 
 // D_mumu over a mu chunk, element (p, s) at mu[p * sp + s * ss]
 template <typename MuT>
-int run_dmumu_t(const PartSource& src, const DmumuArgs& a, const MuT* mu, int64_t sp, int64_t ss, cudaStream_t s)
+int run_dmumu_t(const PartSource& src, const DmumuArgs& a, const MuT* mu, int64_t sp, int64_t ss, cudaStream_t s,
+                int packed = 0)
 {
     pt_ctx* ctx = src.ctx;
     if (a.n <= 0 || a.n_lags <= 0) return PT_OK;
@@ -1116,6 +1117,7 @@ int run_dmumu_t(const PartSource& src, const DmumuArgs& a, const MuT* mu, int64_
             if (a.injection) {
                 DmumuInjection L{};
                 L.mu = mu + p0 * sp; L.sp = sp; L.ss = ss;
+                L.packed = packed; L.first = 1 + lag0;
                 L.n = m; L.nsave = a.nsave; L.lags = a.lags + lag0; L.nl = nl;
                 L.edges = a.edges; L.n_bins = a.n_bins; L.bin_abs = a.bin_abs; L.tile = tile;
                 set_parts(L, (char*)scratch, grid, nl, a.n_bins);
@@ -1151,11 +1153,12 @@ int run_dmumu(pt_ctx* ctx, const DmumuArgs& a, cudaStream_t s)
     return run_dmumu_t<float>(PartSource{ctx, nullptr, 0}, a, a.mu, a.sp, a.ss, s);
 }
 
-int run_dmumu_chunk(pt_ctx* ctx, const DmumuArgs& a, const void* mu, int64_t sp, int64_t ss, int f64, cudaStream_t s)
+int run_dmumu_chunk(pt_ctx* ctx, const DmumuArgs& a, const void* mu, int64_t sp, int64_t ss, int f64, int packed,
+                    cudaStream_t s)
 {
     const PartSource src{ctx, nullptr, 0};
-    return f64 ? run_dmumu_t<double>(src, a, (const double*)mu, sp, ss, s)
-               : run_dmumu_t<float>(src, a, (const float*)mu, sp, ss, s);
+    return f64 ? run_dmumu_t<double>(src, a, (const double*)mu, sp, ss, s, packed)
+               : run_dmumu_t<float>(src, a, (const float*)mu, sp, ss, s, packed);
 }
 
 }  // namespace pt

@@ -422,27 +422,94 @@ __global__ void cell_b_kernel(const R* __restrict__ bx, const R* __restrict__ by
     }
 }
 
-// mu of particles [p0, p0 + m) at every save, written [s][p - p0] (particle
-// fastest, like the device mu cache); one thread per (particle, save),
-// particles fastest so that the phase-space reads coalesce.  B comes from
-// cell records (CELLS) or node records.
-template <typename R, bool CELLS>
-__global__ void __launch_bounds__(256) phase_space_mu_kernel(const R* __restrict__ pos, const R* __restrict__ mom,
-                                                             int64_t row, int64_t comp, int64_t p0, int64_t m,
-                                                             int64_t nsave, const void* __restrict__ Bsrc, pt_grid g,
-                                                             R* __restrict__ mu)
+// Where phase_space_mu_kernel reads B from.
+enum { B_CELLS = 0, B_NODES = 1, B_ARRAYS = 2 };
+struct BSource {
+    const void* records;   // cell or node records
+    const void* arrays[3]; // Bx, By, Bz as they are
+};
+
+// mu of particles [p0, p0 + m) at saves save[r] of `rows` (all saves, or save 0
+// and the lags'), written time-fastest, mu[p - p0][r].  A block takes 32 particles
+// at kPsRows saves: a warp per save, a lane per particle, so that the phase-space
+// reads coalesce; the tile is turned in shared memory, so that the writes do, and
+// the binning reads whole series.
+//
+// With cell records a sample's B is one contiguous record (96 bytes in FP32) at a
+// random place.  The lanes fetch each other's records: 8 (FP64: 16) lanes copy one
+// record to shared memory with 16-byte asynchronous copies, 4 (2) records per warp
+// instruction.  The kernel is bound by the L1's queue of requests that miss, one per
+// line and instruction: with each lane reading its own record in 32-byte loads that
+// queue was full (a third of all stalls) at 41 % of the DRAM bandwidth; now DRAM is
+// 72 % busy.  256^3, 65,536 particles x 801 saves, FP32: 3.20 ms, 2.00 ms now.
+template <typename R>
+constexpr int kPsRows = sizeof(R) == 4 ? 8 : 4;  // 32-byte runs of a particle's mu
+
+__device__ __forceinline__ void copy16_async(void* smem, const void* from)
 {
-    const int64_t total = m * nsave;
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t q = t % m, s = t / m;
-        const R* P = pos + s * row + p0 + q;
-        const R* M = mom + s * row + p0 + q;
-        if constexpr (CELLS)
-            mu[s * m + q] = exact::phase_space_mu_cell<R>(P[0], P[comp], P[2 * comp], M[0], M[comp], M[2 * comp],
-                                                          (const exact::CellB<R>*)Bsrc, g);
-        else
-            mu[s * m + q] = exact::phase_space_mu4<R>(P[0], P[comp], P[2 * comp], M[0], M[comp], M[2 * comp],
-                                                      (const exact::Vec4<R>*)Bsrc, g);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(from)
+                 : "memory");
+}
+
+template <typename R, int SRC>
+__global__ void __launch_bounds__(kWarp* kPsRows<R>)
+    phase_space_mu_kernel(const R* __restrict__ pos, const R* __restrict__ mom, int64_t row, int64_t comp, int64_t p0,
+                          int64_t m, int64_t rows, int64_t nsave, const int64_t* __restrict__ lags, BSource B,
+                          pt_grid g, int64_t pitch, R* __restrict__ mu)
+{
+    constexpr int kChunks = 24 * sizeof(R) / 16;                // 16-byte pieces of a record
+    constexpr int kLanes = kChunks <= 8 ? 8 : 16;               // lanes that copy one
+    constexpr int kRecord = 24 * sizeof(R) + 16;                // padded: a quarter warp's reads hit all banks
+    __shared__ __align__(16) unsigned char s_rec[SRC == B_CELLS ? kPsRows<R> * kWarp * kRecord : 16];
+    __shared__ R tile[kWarp][kPsRows<R> + 1];
+    const int lane = threadIdx.x % kWarp, w = threadIdx.x / kWarp;
+    const int64_t blocks_p = (m + kWarp - 1) / kWarp, blocks_r = (rows + kPsRows<R> - 1) / kPsRows<R>;
+    for (int64_t t = blockIdx.x; t < blocks_p * blocks_r; t += gridDim.x) {
+        const int64_t q = t % blocks_p * kWarp + lane, r0 = t / blocks_p * kPsRows<R>, r = r0 + w;
+        int64_t s = r;
+        if (lags && r > 0 && r < rows) s = lags[r - 1];  // the injection estimator's rows: save 0, then the lags'
+        const bool have = r < rows && q < m && s >= 0 && s < nsave;
+        R v = R(NAN), x[3], p[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            x[k] = have ? pos[s * row + k * comp + p0 + q] : R(NAN);
+            p[k] = have ? mom[s * row + k * comp + p0 + q] : R(NAN);
+        }
+        const bool in = exact::phase_space_inside<R>(x[0], x[1], x[2], p[0], p[1], p[2], g);
+        if constexpr (SRC == B_CELLS) {
+            exact::Cell<R> c{};
+            c.base = -1;
+            if (in)
+                c = exact::locate<R>(x[0], x[1], x[2], (R)g.xmin, (R)g.ymin, (R)g.zmin, (R)g.dx, (R)g.dy, (R)g.dz, g.nx,
+                                     g.ny, g.nz);
+            unsigned char* mine = s_rec + (size_t)w * kWarp * kRecord;
+            const int part = lane % kLanes;
+#pragma unroll
+            for (int k = 0; k < kLanes; ++k) {
+                const int owner = k * (kWarp / kLanes) + lane / kLanes;
+                const int64_t base = __shfl_sync(0xffffffffu, (long long)c.base, owner);
+                if (base >= 0 && part < kChunks)
+                    copy16_async(mine + owner * kRecord + 16 * part,
+                                 (const char*)B.records + base * (int64_t)sizeof(exact::CellB<R>) + 16 * part);
+            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncwarp();
+            if (in) v = exact::cell_mu<R>((const R*)(mine + lane * kRecord), c, p[0], p[1], p[2]);
+        } else if (in) {
+            if constexpr (SRC == B_NODES) {
+                v = exact::phase_space_mu4<R>(x[0], x[1], x[2], p[0], p[1], p[2], (const exact::Vec4<R>*)B.records, g);
+            } else {
+                const R* const b[3] = {(const R*)B.arrays[0], (const R*)B.arrays[1], (const R*)B.arrays[2]};
+                v = exact::phase_space_mu<R>(x[0], x[1], x[2], p[0], p[1], p[2], b, g);
+            }
+        }
+        tile[lane][w] = v;
+        __syncthreads();
+        // thread -> (particle, save), saves fastest
+        const int tp = threadIdx.x / kPsRows<R>, tr = threadIdx.x % kPsRows<R>;
+        const int64_t op = t % blocks_p * kWarp + tp;
+        if (op < m && r0 + tr < rows) mu[op * pitch + r0 + tr] = tile[tp][tr];
+        __syncthreads();
     }
 }
 
@@ -453,53 +520,72 @@ int run_dmumu_phase_space_t(pt_ctx* ctx, const DmumuArgs& a, const R* pos, const
     using V4 = exact::Vec4<R>;
     using CB = exact::CellB<R>;
     const int64_t nodes = g.nx * g.ny * g.nz;
+    // the injection estimator needs save 0 and the lags' saves only
+    const int64_t rows = a.injection ? 1 + (int64_t)a.n_lags : a.nsave;
     // mu chunks of at most 1 GiB
-    const int64_t per = std::max<int64_t>(1, ((int64_t)1 << 30) / ((int64_t)sizeof(R) * a.nsave));
+    const int64_t per = std::max<int64_t>(1, ((int64_t)1 << 30) / ((int64_t)sizeof(R) * rows));
     const int64_t m_max = std::min<int64_t>(a.n, per);
-    const size_t mu_bytes = sizeof(R) * (size_t)m_max * (size_t)a.nsave;
+    const size_t mu_bytes = sizeof(R) * (size_t)m_max * (size_t)rows;
     // B as cell records when they take at most half of the free device
     // memory: a sample then reads one 96-byte (FP32) record instead of 8
     // node records from 4 grid rows, ~4x fewer DRAM bytes on the random
-    // gathers of particles in id order; otherwise as node records
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
-        cudaGetLastError();
-        free_b = 0;
-    }
+    // gathers of particles in id order; otherwise as node records.  Building
+    // the records reads and writes 108 (28) bytes per node, which pays from
+    // about half (an eighth) as many samples as nodes; below, the arrays are read
+    // as they are.
+    const int64_t samples = a.n * rows;
     const size_t cell_bytes = align16(sizeof(CB) * (size_t)nodes);
-    bool cells = cell_bytes + mu_bytes <= free_b / 2;
+    int src = samples >= nodes / 2 ? B_CELLS : (samples >= nodes / 8 ? B_NODES : B_ARRAYS);
     // PTB200_PHASE_SPACE_B = "nodes" or "cells" overrides the choice (same results)
-    if (const char* e = std::getenv("PTB200_PHASE_SPACE_B")) {
-        if (!std::strcmp(e, "nodes")) cells = false;
-        else if (!std::strcmp(e, "cells")) cells = true;
+    const char* want = std::getenv("PTB200_PHASE_SPACE_B");
+    if (want && !std::strcmp(want, "nodes")) {
+        src = B_NODES;
+    } else if (want && !std::strcmp(want, "cells")) {
+        src = B_CELLS;
+    } else if (src == B_CELLS && ctx->scratch[4].bytes < cell_bytes + mu_bytes) {
+        // (asked only when the context does not hold the memory already: the query
+        // can take as long as the whole call)
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+            cudaGetLastError();
+            free_b = 0;
+        }
+        if (cell_bytes + mu_bytes > free_b / 2) src = B_NODES;
     }
-    const size_t b_bytes = cells ? cell_bytes : align16(sizeof(V4) * (size_t)nodes);
+    const size_t b_bytes = src == B_CELLS ? cell_bytes : (src == B_NODES ? align16(sizeof(V4) * (size_t)nodes) : 0);
     void* scratch = nullptr;
     int rc = scratch_get(ctx, 4, b_bytes + mu_bytes, &scratch);
     if (rc) return rc;
     R* mu = (R*)((char*)scratch + b_bytes);
     const int gb = (int)std::min<int64_t>((nodes + 255) / 256, (int64_t)ctx->num_sms * 16);
-    if (cells) {
-        cell_b_kernel<R><<<gb, 256, 0, s>>>((const R*)bfield[0], (const R*)bfield[1], (const R*)bfield[2], g.nx, g.ny,
-                                            g.nz, (CB*)scratch);
+    const R* b[3] = {(const R*)bfield[0], (const R*)bfield[1], (const R*)bfield[2]};
+    if (src == B_CELLS) {
+        cell_b_kernel<R><<<gb, 256, 0, s>>>(b[0], b[1], b[2], g.nx, g.ny, g.nz, (CB*)scratch);
         PT_CHECK_LAUNCH("cell_b_kernel");
-    } else {
-        interleave_b_kernel<R><<<gb, 256, 0, s>>>((const R*)bfield[0], (const R*)bfield[1], (const R*)bfield[2], nodes,
-                                                  (V4*)scratch);
+    } else if (src == B_NODES) {
+        interleave_b_kernel<R><<<gb, 256, 0, s>>>(b[0], b[1], b[2], nodes, (V4*)scratch);
         PT_CHECK_LAUNCH("interleave_b_kernel");
     }
+    const BSource B{scratch, {bfield[0], bfield[1], bfield[2]}};
+    const int64_t* lags = a.injection ? a.lags : nullptr;
     for (int64_t p0 = 0; p0 < a.n; p0 += m_max) {
         const int64_t m = std::min(m_max, a.n - p0);
-        const int64_t total = m * a.nsave;
-        const int blocks = (int)std::min<int64_t>((total + 255) / 256, (int64_t)ctx->num_sms * 32);
-        if (cells)
-            phase_space_mu_kernel<R, true><<<blocks, 256, 0, s>>>(pos, mom, row, comp, p0, m, a.nsave, scratch, g, mu);
+        const int64_t tiles = ((m + kWarp - 1) / kWarp) * ((rows + kPsRows<R> - 1) / kPsRows<R>);
+        const int blocks = (int)std::min<int64_t>(tiles, (int64_t)ctx->num_sms * 64);
+        const int threads = kWarp * kPsRows<R>;
+        if (src == B_CELLS)
+            phase_space_mu_kernel<R, B_CELLS><<<blocks, threads, 0, s>>>(pos, mom, row, comp, p0, m, rows, a.nsave, lags,
+                                                                         B, g, rows, mu);
+        else if (src == B_NODES)
+            phase_space_mu_kernel<R, B_NODES><<<blocks, threads, 0, s>>>(pos, mom, row, comp, p0, m, rows, a.nsave, lags,
+                                                                         B, g, rows, mu);
         else
-            phase_space_mu_kernel<R, false><<<blocks, 256, 0, s>>>(pos, mom, row, comp, p0, m, a.nsave, scratch, g, mu);
+            phase_space_mu_kernel<R, B_ARRAYS><<<blocks, threads, 0, s>>>(pos, mom, row, comp, p0, m, rows, a.nsave,
+                                                                          lags, B, g, rows, mu);
         PT_CHECK_LAUNCH("phase_space_mu_kernel");
         DmumuArgs c = a;
         c.n = m;
-        rc = run_dmumu_chunk(ctx, c, mu, 1, m, sizeof(R) == 8, s);
+        rc = run_dmumu_chunk(ctx, c, mu, rows, 1, sizeof(R) == 8, a.injection, s);
         if (rc) return rc;
     }
     return PT_OK;

@@ -394,8 +394,10 @@ struct DmumuArgs {
     int64_t* pair_n;
 };
 int run_dmumu(pt_ctx* ctx, const DmumuArgs& a, cudaStream_t s);
-// the same over a chunk of Float32 or Float64 mu (a.mu, a.sp, a.ss unused)
-int run_dmumu_chunk(pt_ctx* ctx, const DmumuArgs& a, const void* mu, int64_t sp, int64_t ss, int f64, cudaStream_t s);
+// the same over a chunk of Float32 or Float64 mu (a.mu, a.sp, a.ss unused); packed
+// (injection estimator): the chunk holds save 0 and then the saves of a.lags only
+int run_dmumu_chunk(pt_ctx* ctx, const DmumuArgs& a, const void* mu, int64_t sp, int64_t ss, int f64, int packed,
+                    cudaStream_t s);
 // D_mumu of a phase-space chunk (a.mu, a.sp, a.ss unused): mu reconstructed
 // on the device into a scratch chunk, then binned; component c of save s of
 // particle p at pos/mom + s * row + c * comp + p, elements and B in the

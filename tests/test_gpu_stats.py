@@ -348,3 +348,39 @@ def test_dpp_shapes_and_nan_patterns(cuda, oracle, chunk, nsave, n_lags, pattern
     assert close(g["sum_delta_p_norm2"], o["sum_dpn2"])
     assert close(g["sum_delta_p"], o["sum_dp"], scale=np.sqrt(np.maximum(o["counts"], 1) * o["sum_dp2"]))
     assert close(g["sum_delta_p_norm"], o["sum_dpn"], scale=np.sqrt(np.maximum(o["counts"], 1) * o["sum_dpn2"]))
+
+
+# B read as the arrays are (few samples per node), as cell and as node records; tiles of 32 particles with a remainder;
+# the injection estimator's saves alone, with lags past the series
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("mode", ["sliding", "injection"])
+@pytest.mark.parametrize("b_layout", [None, "cells", "nodes"])
+def test_phase_space_dmumu_b_sources(cuda, oracle, dtype, mode, b_layout, monkeypatch):
+    """As test_phase_space_dmumu_fused_matches_oracle on a grid with more nodes than samples."""
+    torch = cuda
+    monkeypatch.delenv("PTB200_PHASE_SPACE_B", raising=False)
+    if b_layout:
+        monkeypatch.setenv("PTB200_PHASE_SPACE_B", b_layout)
+    from helpers import copy_state, fortran_fields, small_problem
+    pb = small_problem(n=40, n_particles=70)
+    f64 = dtype == np.float64
+    (pos, mom), _ = oracle.push_run(fortran_fields(pb.fields), pb.grid, copy_state(pb.state), np.ones(70, np.uint8),
+                                    pb.dt, 292, 3, cache_mode=2, out_f64=f64)
+    pos[7, 0, 3] = np.nan
+    pos[60:, 1, 4] = np.nan  # a particle that died
+    pos[0, 2, 69] = pb.grid.zmax * 1.01  # outside the box at the first save
+    ff = fortran_fields(pb.fields)[:3]
+    mu = (oracle.reconstruct_mu_f64 if f64 else oracle.reconstruct_mu_f32)(pos, mom, ff, pb.grid)
+    nsave = pos.shape[0]
+    lags = np.concatenate([log_spaced_lag_steps(nsave - 1, 40), [nsave, 5 * nsave]])
+    edges, _ = build_mu_edges_full(0.0, 1.0, 16)
+    o = zero_dmumu(len(lags), 16)
+    oracle.dmumu_accumulate(mu, lags, edges, o, injection=mode == "injection")
+    tdt = torch.float64 if f64 else torch.float32
+    P, M = (torch.as_tensor(v, dtype=tdt, device="cuda") for v in (pos, mom))
+    B = [torch.as_tensor(f, dtype=tdt, device="cuda") for f in pb.fields[:3]]
+    g = S.new_dmumu_accumulators(len(lags), 16, device="cuda")
+    S.process_phase_space_chunk_dmumu(P, M, *B, pb.grid, lags, edges, g["particle_counts"], g["particle_means"],
+                                      g["particle_m2s"], g["pair_sum_squares"], g["pair_counts"], g["dmumu_counts"],
+                                      g["dmumu_sum_delta"], g["dmumu_sum_delta2"], start_mode=mode)
+    check_dmumu({k: v.cpu().numpy() for k, v in g.items()}, o)
