@@ -570,7 +570,8 @@ int pt_fast_state_export(pt_ctx* ctx, const pt_fast_state* st, double* d_x1, dou
     PT_DEVICE_SCOPE(ctx->device);
     if (st->n == 0) return PT_OK;
     if (!(d_x1 && d_x2 && d_x3 && d_p1 && d_p2 && d_p3 && d_alive)) return fail(PT_ERR_ARG, "null state");
-    return launch_fast_export(st, st->field, d_x1, d_x2, d_x3, d_p1, d_p2, d_p3, d_alive, ctx->stream);
+    // the state's values are not changed, but its record memory may be allocated
+    return launch_fast_export(const_cast<pt_fast_state*>(st), st->field, d_x1, d_x2, d_x3, d_p1, d_p2, d_p3, d_alive, ctx->stream);
 }
 
 int pt_fast_state_destroy(pt_fast_state* st)
@@ -587,6 +588,7 @@ int pt_fast_state_destroy(pt_fast_state* st)
     if (st->pid_alt) cudaFree(st->pid_alt);
     if (st->alive_alt) cudaFree(st->alive_alt);
     if (st->sort_tmp) cudaFree(st->sort_tmp);
+    if (st->records) cudaFree(st->records);
     delete st;
     return PT_OK;
 }
@@ -684,6 +686,7 @@ int pt_push_run(pt_ctx* ctx, const pt_field* f, double* x1, double* x2, double* 
             if (n > 0 && (rc = launch_fast_import(fs, f, d[0], d[1], d[2], d[3], d[4], d[5], dal, st))) return rc;
             fs->field = f;
             fs->last_sort = INT64_MIN;
+            fs->sorted = false;
         } else {
             if (fs) {
                 cudaStreamSynchronize(st);

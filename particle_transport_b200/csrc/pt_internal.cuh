@@ -122,6 +122,8 @@ struct pt_fast_state {
     uint8_t* alive_alt = nullptr;
     const pt_field* field = nullptr; // field the state was created against (grid, units)
     int64_t last_sort = INT64_MIN;   // step of the last brick re-sort
+    bool sorted = false;             // the slots have been in brick order since the import
+    void* records = nullptr;         // large states: scatters of a random order go through it (push_fast.cu)
     // scratch for the re-sort
     void* sort_tmp = nullptr;
     size_t sort_tmp_bytes = 0;
@@ -153,9 +155,10 @@ int staged_d2h(const std::vector<HostSeg>& segs, char* stage, size_t chunk, int 
 int64_t count_nonzero(const uint8_t* v, int64_t n);
 
 // ---------------------------------------------------------------- launches
-// Threads per block of a push with one block per SM, at most `most` (a multiple
-// of 128): the fewest that take n particles in as many passes over the chip, in
-// whole warps up to 128 and multiples of 128 (a warp per scheduler) beyond.
+// Threads per block of a push with one block per SM, at most `most`: the fewest
+// whole warps that take n particles in as many passes over the chip.  (The time of
+// a pass goes with the warps of the fullest scheduler, so rounding up to a warp per
+// scheduler gains nothing and leaves SMs without a block.)
 inline int spread_threads(int64_t n, int most)
 {
     int dev = 0, sms = 148;
@@ -163,8 +166,7 @@ inline int spread_threads(int64_t n, int most)
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int64_t per_pass = (int64_t)sms * most, passes = std::max<int64_t>(1, (n + per_pass - 1) / per_pass);
     const int64_t t = std::max<int64_t>(1, (n + sms * passes - 1) / (sms * passes));
-    const int64_t unit = t <= 128 ? 32 : 128;
-    return (int)std::min<int64_t>(most, (t + unit - 1) / unit * unit);
+    return (int)std::min<int64_t>(most, (t + 31) / 32 * 32);
 }
 
 struct PushArgsRef {
@@ -362,7 +364,7 @@ int launch_batch_export(BatchStateDev st0, BatchStateDev st1, const BatchCampaig
                         double* p3, uint8_t* alive, int num_sms, cudaStream_t s);
 int launch_fast_import(pt_fast_state* st, const pt_field* f, const double* x1, const double* x2, const double* x3,
                        const double* p1, const double* p2, const double* p3, const uint8_t* alive, cudaStream_t s);
-int launch_fast_export(const pt_fast_state* st, const pt_field* f, double* x1, double* x2, double* x3, double* p1,
+int launch_fast_export(pt_fast_state* st, const pt_field* f, double* x1, double* x2, double* x3, double* p1,
                        double* p2, double* p3, uint8_t* alive, cudaStream_t s);
 int fast_sort(pt_ctx* ctx, pt_fast_state* st, const pt_field* f, cudaStream_t s);
 

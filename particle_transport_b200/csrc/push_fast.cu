@@ -387,6 +387,23 @@ __global__ void fast_import_kernel(const double* __restrict__ x1, const double* 
     }
 }
 
+// SI state of a slot (positions in cells xc, p/(mc) pc, |p/(mc)|^2 P2)
+struct SiState {
+    double x[3], p[3];
+};
+__device__ __forceinline__ SiState si_state(const double (&xc)[3], const float (&pc)[3], double P2, double xmin,
+                                            double ymin, double zmin, double dx, double dy, double dz)
+{
+    SiState r;
+    r.x[0] = xmin + xc[0] * dx;
+    r.x[1] = ymin + xc[1] * dy;
+    r.x[2] = zmin + xc[2] * dz;
+    const double px = pc[0], py = pc[1], pz = pc[2];
+    const double sc = sqrt(P2 / (px * px + py * py + pz * pz)) * (M_P * C_LIGHT);
+    r.p[0] = px * sc; r.p[1] = py * sc; r.p[2] = pz * sc;
+    return r;
+}
+
 __global__ void fast_export_kernel(const double* __restrict__ xs, const float* __restrict__ ps,
                                    const double* __restrict__ p2s, const int32_t* __restrict__ pid,
                                    const uint8_t* __restrict__ as, int64_t n, double xmin, double ymin, double zmin,
@@ -395,13 +412,96 @@ __global__ void fast_export_kernel(const double* __restrict__ xs, const float* _
 {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t q = pid[i];
-        x1[q] = xmin + xs[i] * dx;
-        x2[q] = ymin + xs[n + i] * dy;
-        x3[q] = zmin + xs[2 * n + i] * dz;
-        const double px = ps[i], py = ps[n + i], pz = ps[2 * n + i];
-        const double sc = sqrt(p2s[i] / (px * px + py * py + pz * pz)) * (M_P * C_LIGHT);
-        p1[q] = px * sc; p2[q] = py * sc; p3[q] = pz * sc;
+        const SiState r = si_state({xs[i], xs[n + i], xs[2 * n + i]}, {ps[i], ps[n + i], ps[2 * n + i]}, p2s[i], xmin,
+                                   ymin, zmin, dx, dy, dz);
+        x1[q] = r.x[0]; x2[q] = r.x[1]; x3[q] = r.x[2];
+        p1[q] = r.p[0]; p2[q] = r.p[1]; p3[q] = r.p[2];
         alive[q] = as[i];
+    }
+}
+
+// Many particles leave their slots for places of a random order (their ids, or
+// the slots of a first sort) through records: pack writes each particle as one
+// 64-byte record at its place, unpack reads the records in order and writes the
+// arrays coalesced.  Scattered directly, each of the nine values costs a 32-byte
+// sector that DRAM reads and writes back: exporting 16.7M particles took 4.7 ms,
+// with records 0.9.  The records hold a window of kRecordWindow places, so that the
+// memory is bounded; each window's pack reads all places.  Below kRecordMin
+// particles the arrays of the direct scatter stay in L2, where its sectors merge.
+struct alignas(32) StateRecord {
+    double x[3], p2;
+    float p[3];
+    int32_t pid;
+    uint32_t alive;
+    uint32_t pad[3];
+};
+static_assert(sizeof(StateRecord) == 64, "two sectors");
+constexpr int64_t kRecordWindow = 2 << 20;  // 128 MB
+constexpr int64_t kRecordMin = 1 << 21;
+
+// 32-byte store (sm_100 256-bit vector store; the address is 32-byte aligned)
+__device__ __forceinline__ void stg256(void* p, const uint32_t w[8])
+{
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]),
+                 "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
+}
+
+// place[i] - base: the record of slot i's particle, when below count
+__global__ void record_pack_kernel(const uint32_t* __restrict__ place, uint32_t base, uint32_t count, int64_t n,
+                                   const double* __restrict__ xs, const float* __restrict__ ps,
+                                   const double* __restrict__ p2s, const int32_t* __restrict__ pid,
+                                   const uint8_t* __restrict__ as, StateRecord* __restrict__ out)
+{
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t d = place[i] - base;
+        if (d >= count) continue;
+        const double v[4] = {xs[i], xs[n + i], xs[2 * n + i], p2s[i]};
+        uint32_t w[8];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            w[2 * k] = (uint32_t)__double2loint(v[k]);
+            w[2 * k + 1] = (uint32_t)__double2hiint(v[k]);
+        }
+        stg256(out + d, w);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) w[k] = __float_as_uint(ps[k * n + i]);
+        w[3] = (uint32_t)pid[i];
+        w[4] = as[i];
+        w[5] = w[6] = w[7] = 0u;
+        stg256((char*)(out + d) + 32, w);
+    }
+}
+
+__global__ void record_export_kernel(const StateRecord* __restrict__ rec, int64_t count, double xmin, double ymin,
+                                     double zmin, double dx, double dy, double dz, double* x1, double* x2, double* x3,
+                                     double* p1, double* p2, double* p3, uint8_t* alive)
+{
+    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < count;
+         q += (int64_t)gridDim.x * blockDim.x) {
+        const StateRecord v = rec[q];
+        const SiState r = si_state({v.x[0], v.x[1], v.x[2]}, {v.p[0], v.p[1], v.p[2]}, v.p2, xmin, ymin, zmin, dx, dy,
+                                   dz);
+        x1[q] = r.x[0]; x2[q] = r.x[1]; x3[q] = r.x[2];
+        p1[q] = r.p[0]; p2[q] = r.p[1]; p3[q] = r.p[2];
+        alive[q] = (uint8_t)v.alive;
+    }
+}
+
+// records -> slots [d0, d0 + count) of a state of n
+__global__ void record_unpack_kernel(const StateRecord* __restrict__ rec, int64_t d0, int64_t count, int64_t n,
+                                     double* __restrict__ xs, float* __restrict__ ps, double* __restrict__ p2s,
+                                     int32_t* __restrict__ pid, uint8_t* __restrict__ as)
+{
+    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < count;
+         q += (int64_t)gridDim.x * blockDim.x) {
+        const StateRecord v = rec[q];
+        const int64_t d = d0 + q;
+        xs[d] = v.x[0]; xs[n + d] = v.x[1]; xs[2 * n + d] = v.x[2];
+        ps[d] = v.p[0]; ps[n + d] = v.p[1]; ps[2 * n + d] = v.p[2];
+        p2s[d] = v.p2;
+        pid[d] = v.pid;
+        as[d] = (uint8_t)v.alive;
     }
 }
 
@@ -637,6 +737,23 @@ __global__ void __launch_bounds__(kScatterBlock) sort_scatter_block_kernel(
     ad[d] = sh.alive[q];
 }
 
+// The sorted slot of every particle, for a scatter through records.
+__global__ void __launch_bounds__(kScatterBlock) sort_place_kernel(uint32_t* cursor,
+                                                                   const uint32_t* __restrict__ tile_off, int64_t n,
+                                                                   const uint32_t* __restrict__ offs, int nx, int ny,
+                                                                   int nz, uint32_t dead_key,
+                                                                   const double* __restrict__ xs,
+                                                                   const uint8_t* __restrict__ as,
+                                                                   uint32_t* __restrict__ place)
+{
+    __shared__ RunScratch<kScatterBlock> run;
+    const int64_t i0 = (int64_t)blockIdx.x * kScatterBlock, i = i0 + threadIdx.x;
+    const uint32_t key =
+        i < n ? brick_key(xs[i], xs[n + i], xs[2 * n + i], as[i], offs, nx, ny, nz, dead_key) : kPastEnd;
+    const BlockRun r = block_runs(key, cursor, tile_off, run);
+    if (r.dest >= 0) place[i0 + r.src] = (uint32_t)r.dest;
+}
+
 // ---- brick sort of an FP64 SI state (the FP64 push over BRICK_F64 fields):
 // xs = [6][n] (x1, x2, x3, p1, p2, p3), pid, alive.  The bucket is the
 // brick of the cell holding the position; it only orders the slots.
@@ -763,9 +880,7 @@ int launch_push_fast_shape(const PushArgsFast& a, cudaStream_t s, int cap_per_sm
 // the same: 23.0 with 512, 18.9 with 768, 17.3 with 1024 (half the loads: fewer
 // registers and L1 wavefronts); FP32, 256^3, 1M particles: 2.64 ms with 2 x 256,
 // 2.66 with 512, 2.85 with 640.
-// Few particles are spread over all SMs: the fewest threads that take them in as
-// many passes, in whole warps up to 4 and whole warps per scheduler beyond (576
-// threads take 22.9 ms where 512 take 20.9).
+// Few particles are spread over all SMs (spread_threads).
 template <int LAYOUT, int BLOCK>
 int launch_push_fast_auto(const PushArgsFast& a, cudaStream_t s)
 {
@@ -920,11 +1035,47 @@ int launch_fast_import(pt_fast_state* st, const pt_field* f, const double* x1, c
     return PT_OK;
 }
 
-int launch_fast_export(const pt_fast_state* st, const pt_field* f, double* x1, double* x2, double* x3, double* p1,
-                       double* p2, double* p3, uint8_t* alive, cudaStream_t s)
+// The state's own record memory -- kRecordWindow records, then a place per particle
+// -- or null where records do not pay or it is not to be had (the direct scatter
+// needs none).  Allocated on first use, but not inside a stream capture.
+static StateRecord* record_window(pt_fast_state* st, cudaStream_t s)
+{
+    if (st->n < kRecordMin) return nullptr;
+    if (!st->records) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        const size_t bytes = sizeof(StateRecord) * (size_t)std::min(st->n, kRecordWindow) + sizeof(uint32_t) * st->n;
+        if (cudaMalloc(&st->records, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            st->records = nullptr;
+        }
+    }
+    return (StateRecord*)st->records;
+}
+
+int launch_fast_export(pt_fast_state* st, const pt_field* f, double* x1, double* x2, double* x3,
+                       double* p1, double* p2, double* p3, uint8_t* alive, cudaStream_t s)
 {
     const pt_grid& g = f->grid;
-    fast_export_kernel<<<grid_for(st->n, 256, st->ctx->num_sms), 256, 0, s>>>(
+    const int sms = st->ctx->num_sms;
+    if (StateRecord* rec = record_window(st, s)) {
+        for (int64_t d0 = 0; d0 < st->n; d0 += kRecordWindow) {
+            const int64_t c = std::min(kRecordWindow, st->n - d0);
+            record_pack_kernel<<<grid_for(st->n, 256, sms), 256, 0, s>>>((const uint32_t*)st->pid, (uint32_t)d0,
+                                                                         (uint32_t)c, st->n, st->x, st->p, st->p2,
+                                                                         st->pid, st->alive, rec);
+            PT_CHECK_LAUNCH("record_pack_kernel");
+            record_export_kernel<<<grid_for(c, 256, sms), 256, 0, s>>>(rec, c, g.xmin, g.ymin, g.zmin, g.dx, g.dy, g.dz,
+                                                                       x1 + d0, x2 + d0, x3 + d0, p1 + d0, p2 + d0,
+                                                                       p3 + d0, alive + d0);
+            PT_CHECK_LAUNCH("record_export_kernel");
+        }
+        return PT_OK;
+    }
+    fast_export_kernel<<<grid_for(st->n, 256, sms), 256, 0, s>>>(
         st->x, st->p, st->p2, st->pid, st->alive, st->n, g.xmin, g.ymin, g.zmin, g.dx, g.dy, g.dz, x1, x2, x3, p1,
         p2, p3, alive);
     PT_CHECK_LAUNCH("fast_export_kernel");
@@ -985,15 +1136,38 @@ int fast_sort(pt_ctx* ctx, pt_fast_state* st, const pt_field* f, cudaStream_t s)
     PT_CHECK_LAUNCH("sort_scan_tiles_kernel");
     sort_scan_top_kernel<<<1, 1024, 0, s>>>(tile_off, tiles, nullptr);
     PT_CHECK_LAUNCH("sort_scan_top_kernel");
-    sort_scatter_block_kernel<<<(unsigned)((n + kScatterBlock - 1) / kScatterBlock), kScatterBlock, 0, s>>>(
-        cur, tile_off, n, f->offs, nx, ny, nz, nb, st->x, st->p, st->p2, st->pid, st->alive, st->x_alt, st->p_alt,
-        st->p2_alt, st->pid_alt, st->alive_alt);
-    PT_CHECK_LAUNCH("sort_scatter_block_kernel");
+    const unsigned sb = (unsigned)((n + kScatterBlock - 1) / kScatterBlock);
+    // a state's first sort finds its particles in no order: 16.7M particles take
+    // 4.9 ms scattered directly.  Later ones find them in runs (0.9 ms).
+    StateRecord* rec = st->sorted ? nullptr : record_window(st, s);
+    if (rec) {
+        uint32_t* place = (uint32_t*)(rec + std::min(n, kRecordWindow));
+        sort_place_kernel<<<sb, kScatterBlock, 0, s>>>(cur, tile_off, n, f->offs, nx, ny, nz, nb, st->x, st->alive,
+                                                       place);
+        PT_CHECK_LAUNCH("sort_place_kernel");
+        for (int64_t d0 = 0; d0 < n; d0 += kRecordWindow) {
+            const int64_t c = std::min(kRecordWindow, n - d0);
+            record_pack_kernel<<<grid_for(n, 256, ctx->num_sms), 256, 0, s>>>(place, (uint32_t)d0, (uint32_t)c, n,
+                                                                              st->x, st->p, st->p2, st->pid, st->alive,
+                                                                              rec);
+            PT_CHECK_LAUNCH("record_pack_kernel");
+            record_unpack_kernel<<<grid_for(c, 256, ctx->num_sms), 256, 0, s>>>(rec, d0, c, n, st->x_alt, st->p_alt,
+                                                                                st->p2_alt, st->pid_alt,
+                                                                                st->alive_alt);
+            PT_CHECK_LAUNCH("record_unpack_kernel");
+        }
+    } else {
+        sort_scatter_block_kernel<<<sb, kScatterBlock, 0, s>>>(cur, tile_off, n, f->offs, nx, ny, nz, nb, st->x, st->p,
+                                                               st->p2, st->pid, st->alive, st->x_alt, st->p_alt,
+                                                               st->p2_alt, st->pid_alt, st->alive_alt);
+        PT_CHECK_LAUNCH("sort_scatter_block_kernel");
+    }
     std::swap(st->x, st->x_alt);
     std::swap(st->p, st->p_alt);
     std::swap(st->p2, st->p2_alt);
     std::swap(st->pid, st->pid_alt);
     std::swap(st->alive, st->alive_alt);
+    st->sorted = true;
     return PT_OK;
 }
 

@@ -361,3 +361,37 @@ def test_fp64_push_particle_counts(cuda, storage, n):
     assert np.array_equal(mu_o, col.mu, equal_nan=True)
     for k in R.KEYS:
         assert np.array_equal(st_o[k], st_g[k]), k
+
+
+def test_large_state_through_records_bit_identical(cuda):
+    """Above 2^21 particles the first sort and the export go through records, here in two windows (the second of 5
+    places): the exported state is that of the unsorted slots, and of a small state's direct scatter, bit for bit."""
+    torch = cuda
+    n = (1 << 21) + 5
+    pb = small_problem(n=16, n_particles=1000, u_over_c=1e-4, energy_GeV=3.0)
+    st = {k: np.resize(v, n) * (1.0 + 1e-7 * (np.arange(n) // 1000)) for k, v in pb.state.items()}
+    for k in ("x1", "x2", "x3"):
+        st[k] = np.mod(st[k], pb.grid.xmax)
+    alive = np.ones(n, np.uint8)
+    alive[::7] = 0
+    fl = FieldLibrary(pb.fields, pb.grid, "brick_bf16")
+    params = R.push_params(pb.dt, 100, 4, cache="none", precision="f32")
+    outs = []
+    for sort in (False, True):
+        ens = R.FastEnsemble(fl, st, alive)
+        if sort:
+            ens.sort()
+        ens.advance(params, 0, 3)
+        if sort:
+            ens.sort()  # a later sort scatters directly
+        outs.append(ens.export())
+        ens.close()
+    tail = slice(n - 1500, n)
+    small = R.FastEnsemble(fl, {k: v[tail].copy() for k, v in st.items()}, alive[tail].copy())
+    small.advance(params, 0, 3)
+    outs.append(small.export())
+    (a, al), (b, bl), (c, cl) = outs
+    for k in R.KEYS:
+        assert torch.equal(a[k], b[k]), k
+        assert torch.equal(a[k][n - 1500:], c[k]), k
+    assert torch.equal(al, bl) and torch.equal(al[n - 1500:], cl) and torch.equal(al.cpu(), torch.as_tensor(alive))
