@@ -49,6 +49,7 @@ struct pt_batch {
     int stage_next = 0;
     BatchCampaignDev* d_stage = nullptr;
     std::vector<BatchTile> tile_scratch;
+    std::vector<int32_t> bucket_scratch;
 };
 
 namespace {
@@ -88,6 +89,39 @@ void drop_graphs(pt_batch* b)
     b->graph_dirty = true;
 }
 
+int64_t campaign_tiles(const BatchCampaignDev& C) { return (C.n + kBatchTile - 1) / kBatchTile; }
+
+// The tile table: the campaigns side by side, each at the same fraction of its
+// slots.  A sorted campaign sweeps its field in brick order, so campaigns that
+// share a field then read a brick at about the same time, and one passage of the
+// field through L2 serves all of them (one campaign after another, six campaigns
+// on a 537 MB field read it from DRAM six times an epoch: 5.3 of 6.5 TB/s); and
+// tiles that wait for DRAM run beside tiles that do not.  Tile k of T goes to
+// bucket (2 k + 1) most / (2 T) of `most`, so a bucket holds at most one tile of
+// a campaign; a counting sort over the buckets, linear in the tiles.
+void interleave_tiles(pt_batch* b, int64_t total, int64_t most)
+{
+    std::vector<BatchTile>& tiles = b->tile_scratch;
+    std::vector<int32_t>& first = b->bucket_scratch;
+    tiles.resize((size_t)total);
+    first.assign((size_t)most + 1, 0);
+    auto each = [&](auto&& fn) {
+        for (int c = 0; c < b->max_camps; ++c) {
+            const BatchCampaignDev& C = b->h_camps[c];
+            if (!C.active || !C.running) continue;
+            const int64_t T = campaign_tiles(C);
+            for (int64_t k = 0; k < T; ++k) fn(c, C, k, (2 * k + 1) * most / (2 * T));
+        }
+    };
+    each([&](int, const BatchCampaignDev&, int64_t, int64_t bucket) { ++first[(size_t)bucket + 1]; });
+    for (size_t i = 1; i < first.size(); ++i) first[i] += first[i - 1];
+    each([&](int c, const BatchCampaignDev& C, int64_t k, int64_t bucket) {
+        const int64_t s = k * kBatchTile;
+        tiles[(size_t)first[(size_t)bucket]++] =
+            BatchTile{c, (int32_t)std::min<int64_t>(kBatchTile, C.n - s), C.slot0 + s};
+    });
+}
+
 // Recompute sort buckets and tile table after the campaign set changed and
 // upload them behind the epochs already enqueued, without waiting for them.
 // The step counters are advanced on the device by every epoch, so the host
@@ -99,15 +133,16 @@ int rebuild_tables(pt_batch* b, int fresh)
 {
     int64_t key = 0;
     std::vector<BatchTile>& tiles = b->tile_scratch;
-    tiles.clear();
+    int64_t total = 0, most = 0;  // tiles of all running campaigns, of the largest
     for (int c = 0; c < b->max_camps; ++c) {
         BatchCampaignDev& C = b->h_camps[c];
         if (!C.active || !C.running) continue;
         C.key_base = key;
         key += C.n_bricks + 1;
-        for (int64_t s = 0; s < C.n; s += kBatchTile)
-            tiles.push_back(BatchTile{c, (int32_t)std::min<int64_t>(kBatchTile, C.n - s), C.slot0 + s});
+        total += campaign_tiles(C);
+        most = std::max(most, campaign_tiles(C));
     }
+    interleave_tiles(b, total, most);
     if (key > UINT32_MAX) return fail(PT_ERR_ARG, "too many sort buckets in the batch");
     if (key > b->hist_cap) {
         const int64_t want = std::max<int64_t>(key, 2 * b->hist_cap);

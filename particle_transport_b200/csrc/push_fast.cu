@@ -1265,12 +1265,12 @@ __global__ void __launch_bounds__(BLOCK, 1) push_batch_kernel(BatchLaunch L)
             }
             __syncthreads();
             if (threadIdx.x == 0) s_camp = T.campaign;
-            if (s_a.fld.offs != s_loaded) {
+            if (!s_a.fld.morton && s_a.fld.offs != s_loaded) {
                 const int tot = (int)(s_a.fld.nx + s_a.fld.ny + s_a.fld.nz);
                 for (int i = threadIdx.x; i < tot; i += blockDim.x) s_offs[i] = s_a.fld.offs[i];
             }
             __syncthreads();
-            if (threadIdx.x == 0) s_loaded = s_a.fld.offs;
+            if (threadIdx.x == 0 && !s_a.fld.morton) s_loaded = s_a.fld.offs;
         }
         const int64_t sb = s_begin, se = s_end;
         if (sb >= se) continue;
