@@ -10,7 +10,7 @@
 // loop is 4 starts of one bin against 8 lags of one set, and every lane keeps
 // (sum dmu, sum dmu^2) of its NS lags for the current bin in registers.  At the
 // end of a bin the four starts' sums are added across lanes and flushed to the
-// CTA's shared (bin, lag) sums.  Compared with one lag per lane: 55 lags fill 56
+// CTA's (bin, lag) partials.  Compared with one lag per lane: 55 lags fill 56
 // of 56 lane columns instead of 55 of 64, and the start's index, value and
 // float-to-double conversion are shared by all NS sets.
 //
@@ -23,12 +23,10 @@
 // partner and counts pairs.
 //
 // What bounds it: instruction issue (60 % busy at 16 warps per SM) with the
-// shared-memory pipe (68 %) and the conversion pipe (48 %) close behind; a pair
+// shared-memory pipe (67 %) and the conversion pipe (48 %) close behind; a pair
 // row costs an address add, a load, a conversion, two adds and an FMA.  131,072
-// x 4001 saves x 55 lags x 50 bins: 28.2 ms with one lag per lane, 16.1 ms now
-// (1.5e12 pairs/s); 4096 x 801 x 19 x 20: 263 us, 147 us now.  512 threads with 128
-// registers: with 80 (768 threads) the pair loop of 7 sets spills and the same
-// call takes 20.5 ms.
+// x 4001 saves x 55 lags x 50 bins: 28.2 ms with one lag per lane, 15.1 ms now
+// (1.6e12 pairs/s); 4096 x 801 x 19 x 20: 263 us, 147 us now.
 //
 // Injection estimator (dmumu_injection_kernel): only saves 0 and the lags are
 // read: 524,287 particles x 29 of 801 saves take 139 us; staging every save as
@@ -53,9 +51,14 @@ constexpr int kWarp = 32;
 constexpr int kLagLanes = 8;    // lags of a set: lanes of a row along the lag axis
 constexpr int kStartLanes = 4;  // starts of a row
 constexpr int kMaxSets = 8;     // lag sets of a warp (64 lags)
-constexpr int kMaxThreads = 512;
+// Threads of a CTA: the accumulators of NS sets decide the registers of a thread.
+// 7 sets, 131,072 x 4001 saves: 15.1 ms with 512 threads, 18.1 with 384, 21.3 with
+// 640 (96 registers, spilled); 4 sets, 65,536 x 801: 1.33 ms with 512, 1.25 with 640,
+// 1.40 with 768.
+__host__ __device__ constexpr int max_threads(int ns) { return ns <= 4 ? 640 : 512; }
 constexpr int kBatch = 4;       // saves that a thread stages side by side
-constexpr int kFlushCost = 12;  // starts whose pairs cost as much as the end of a bin
+constexpr int kKeep = 16;       // saves per thread whose bucket and rank stay in registers until the list is written
+constexpr int kFlushCost = 28;  // starts whose pairs cost as much as the end of a bin, its last rows included
 constexpr int kMaxSlots = 15;   // one named barrier per slot (barrier 0 is __syncthreads)
 
 struct WelfordPart {
@@ -149,7 +152,7 @@ struct DmumuLaunch {
     char* gslots;              // global staging of the slots' series and lists, when they do not fit on chip
     size_t gslot_bytes;
     // per-CTA outputs
-    unsigned long long* part_cnt;  // [grid][nl][n_bins]
+    unsigned long long* part_cnt;  // [grid][n_bins][nl]
     double* part_sd;
     double* part_sd2;
     WelfordPart* part_w;           // [grid][nl]
@@ -176,15 +179,12 @@ constexpr unsigned kFar = 0x7fffffffu;
 
 // shared memory of the CTA ahead of the slots
 struct DmumuFixed {
-    size_t sd2, hist2, edges, lag, sorted, rank, lane, total;
+    size_t edges, lag, sorted, rank, lane, total;  // hist2 comes first
 };
 __host__ __device__ inline DmumuFixed dmumu_fixed(int nl, int n_bins, int mu_bytes, int lanes, int ktab)
 {
     DmumuFixed f;
-    const size_t acc = (size_t)nl * n_bins * sizeof(double);
-    f.sd2 = acc;
-    f.hist2 = 2 * acc;
-    f.edges = up16(f.hist2 + sizeof(unsigned) * (size_t)n_bins * (nl + 1));
+    f.edges = up16(sizeof(unsigned) * (size_t)n_bins * (nl + 1));
     f.lag = up16(f.edges + (size_t)mu_bytes * (n_bins + 1));
     f.sorted = f.lag + sizeof(int) * nl;
     f.rank = f.sorted + sizeof(int) * nl;
@@ -192,7 +192,7 @@ __host__ __device__ inline DmumuFixed dmumu_fixed(int nl, int n_bins, int mu_byt
     f.total = up16(up16(f.lane + sizeof(int) * lanes) + ktab);
     return f;
 }
-// shared memory of a slot: series | list | hist[B] | cur[B + 1], next[B] |
+// shared memory of a slot: series | list | hist[2][B] | cur[B + 1], next[B] |
 // welford[nl] | tot_sd2[nl] | tot_c[nl] | nfin, with B = 2 (nb + 1) buckets
 // (series and list elsewhere when GLOBAL)
 struct DmumuSlot {
@@ -203,7 +203,7 @@ __host__ __device__ inline DmumuSlot dmumu_slot(int mode, int64_t nsave, int mu_
     DmumuSlot o;
     o.list = mode == SLOT_GLOBAL ? 0 : up16((size_t)nsave * slot_stride(mode, mu_bytes));
     o.hist = mode == SLOT_GLOBAL ? 0 : o.list + up16((size_t)nsave * 2);
-    o.cur = o.hist + sizeof(int) * 2 * (n_bins + 1);
+    o.cur = o.hist + sizeof(int) * 4 * (n_bins + 1);
     o.welford = up16(o.cur + sizeof(int) * (4 * (n_bins + 1) + 1));
     o.tot = o.welford + sizeof(WelfordPart) * nl;
     o.totc = o.tot + sizeof(double) * nl;
@@ -267,8 +267,8 @@ template <typename MuT, typename IdxT, int NS, int MODE, bool TEST>
 __device__ __forceinline__ void dmumu_pairs(const MuT* series,
                                             const IdxT* list, const int* cur, bool clear_ok, int nb, int nl, int b,
                                             int r0, int r1, int end_save, const unsigned (&off)[NS], int lane,
-                                            const int* lane_lag, double* acc_sd, double* acc_sd2,
-                                            unsigned long long* cnt_out, double* tot_sd2, int* tot_c)
+                                            const int* lane_lag, double* out_sd, double* out_sd2,
+                                            unsigned long long* out_cnt, double* tot_sd2, int* tot_c)
 {
     constexpr unsigned kStride = slot_stride(MODE, sizeof(MuT));
     constexpr int kOwn = (NS + kStartLanes - 1) / kStartLanes, kShort = NS - long_sets(NS);
@@ -348,11 +348,14 @@ __device__ __forceinline__ void dmumu_pairs(const MuT* series,
                 ownc[q] += fc;
             }
             if (b < nb && mine[q] >= 0) {
+                // straight to the CTA's partials in L2: reductions that nothing
+                // waits for (a shared-memory double add is a compare-and-swap
+                // loop: 2,200 cycles a flush)
                 const int ai = b * nl + mine[q];  // [bin][lag]
-                atomicAdd(&acc_sd[ai], fd);
-                atomicAdd(&acc_sd2[ai], fq);
+                atomicAdd(&out_sd[ai], fd);
+                atomicAdd(&out_sd2[ai], fq);
                 if constexpr (TEST)
-                    if (fc > 0) atomicAdd(&cnt_out[(int64_t)mine[q] * nb + b], (unsigned long long)fc);
+                    if (fc > 0) atomicAdd(&out_cnt[ai], (unsigned long long)fc);
             }
         }
         e = e1;
@@ -367,7 +370,7 @@ __device__ __forceinline__ void dmumu_pairs(const MuT* series,
 }
 
 template <typename MuT, int NS, int MODE>
-__global__ void __launch_bounds__(kMaxThreads, 1) dmumu_kernel(DmumuLaunch a)
+__global__ void __launch_bounds__(max_threads(NS), 1) dmumu_kernel(DmumuLaunch a)
 {
     using IdxT = std::conditional_t<MODE == SLOT_GLOBAL, uint32_t, uint16_t>;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -375,9 +378,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) dmumu_kernel(DmumuLaunch a)
     const int sets = a.groups * NS;
     const int ktab_bytes = MODE == SLOT_REP ? nsave + 1 : 0;
     const DmumuFixed F = dmumu_fixed(nl, nb, sizeof(MuT), sets * kLagLanes, ktab_bytes);
-    double* acc_sd = (double*)smem;  // [bin][lag]
-    double* acc_sd2 = (double*)(smem + F.sd2);
-    unsigned* hist2 = (unsigned*)(smem + F.hist2);  // [bin][k]: starts that reach k lags
+    unsigned* hist2 = (unsigned*)smem;  // [bin][k]: starts that reach k lags
     MuT* s_edge = (MuT*)(smem + F.edges);
     int* s_lag = (int*)(smem + F.lag);        // lag in saves, nsave when no pair exists
     int* s_sorted = (int*)(smem + F.sorted);  // ascending
@@ -385,13 +386,16 @@ __global__ void __launch_bounds__(kMaxThreads, 1) dmumu_kernel(DmumuLaunch a)
     int* s_lane = (int*)(smem + F.lane);      // lag of (set, lag lane), -1: idle
     uint8_t* ktab = smem + up16(F.lane + sizeof(int) * (size_t)sets * kLagLanes);  // [x]: lags below x (REP)
     const int64_t cta = blockIdx.x;
-    unsigned long long* cnt_out = a.part_cnt + cta * nl * nb;
+    unsigned long long* out_cnt = a.part_cnt + cta * nl * nb;  // [bin][lag]
+    double* out_sd = a.part_sd + cta * nl * nb;
+    double* out_sd2 = a.part_sd2 + cta * nl * nb;
 
     for (int i = threadIdx.x; i < nl * nb; i += blockDim.x) {
-        acc_sd[i] = 0.0;
-        acc_sd2[i] = 0.0;
-        cnt_out[i] = 0ull;
+        out_cnt[i] = 0ull;
+        out_sd[i] = 0.0;
+        out_sd2[i] = 0.0;
     }
+    __threadfence();
     for (int i = threadIdx.x; i < nb * (nl + 1); i += blockDim.x) hist2[i] = 0u;
     for (int i = threadIdx.x; i <= nb; i += blockDim.x) s_edge[i] = edge_up(a.edges[i], MuT());
     for (int i = threadIdx.x; i < sets * kLagLanes; i += blockDim.x) s_lane[i] = -1;
@@ -456,14 +460,15 @@ __global__ void __launch_bounds__(kMaxThreads, 1) dmumu_kernel(DmumuLaunch a)
     IdxT* list = MODE == SLOT_GLOBAL ? (IdxT*)(gb + up16(sizeof(MuT) * (size_t)a.nsave)) : (IdxT*)(sb + O.list);
     // buckets of the start list: 2 b + (0: clear, 1: not) of bin b
     const int nbk = 2 * (nb + 1);
-    int* hist = (int*)(sb + O.hist);     // starts per bucket
+    int* hist = (int*)(sb + O.hist);     // starts per bucket whose rank a thread keeps, then the others
+    int* hist_r = hist + nbk;
     int* cur = (int*)(sb + O.cur);       // first list entry of each bucket; cur[nbk] = all
-    int* next = cur + nbk + 1;           // next free list entry of each bucket
+    int* next = cur + nbk + 1;           // next free entry for a start whose rank was not kept
     WelfordPart* wel = (WelfordPart*)(sb + O.welford);
     double* tot_sd2 = (double*)(sb + O.tot);
     int* tot_c = (int*)(sb + O.totc);
     int* nfin_s = (int*)(sb + O.nfin);
-    for (int i = st; i < nbk; i += T) hist[i] = 0;
+    for (int i = st; i < 2 * nbk; i += T) hist[i] = 0;
     for (int i = st; i < nl; i += T) {
         wel[i] = WelfordPart{0, 0.0, 0.0, 0.0, 0};
         tot_sd2[i] = 0.0;
@@ -486,12 +491,12 @@ __global__ void __launch_bounds__(kMaxThreads, 1) dmumu_kernel(DmumuLaunch a)
         // ---- stage the series and count the starts per bucket, kBatch saves of a
         // thread side by side (one after another they are a chain of a load, a
         // conversion, two shared reads and an atomic each)
+        uint32_t pk[kKeep];  // bucket << 16 | rank within it, ~0: not a start
         {
             int bad = nsave;
             const MuT* q = row;
-            for (int s0 = st; s0 < nsave; s0 += kBatch * T, q += kBatch * hop) {
+            auto stage = [&](int s0, int (&b)[kBatch]) {
                 MuT v[kBatch];
-                int b[kBatch];
 #pragma unroll
                 for (int i = 0; i < kBatch; ++i) v[i] = s0 + i * T < nsave ? q[i * hop] : MuT(NAN);
                 bins_of(v, E, b);
@@ -505,9 +510,25 @@ __global__ void __launch_bounds__(kMaxThreads, 1) dmumu_kernel(DmumuLaunch a)
                         if (b[i] < 0) bad = min(bad, s);
                     }
                 }
+                q += kBatch * hop;
+            };
+#pragma unroll
+            for (int i0 = 0; i0 < kKeep; i0 += kBatch) {
+                if (i0 * T >= nsave) break;
+                int b[kBatch];
+                stage(i0 * T + st, b);
+#pragma unroll
+                for (int i = 0; i < kBatch; ++i) {
+                    const int k = 2 * b[i] + ((i0 + i) * T + st >= clear_end);
+                    pk[i0 + i] = b[i] < 0 ? 0xffffffffu : (uint32_t)k << 16 | (uint32_t)atomicAdd(&hist[k], 1);
+                }
+            }
+            for (int s0 = kKeep * T + st; s0 < nsave; s0 += kBatch * T) {
+                int b[kBatch];
+                stage(s0, b);
 #pragma unroll
                 for (int i = 0; i < kBatch; ++i)
-                    if (b[i] >= 0) atomicAdd(&hist[2 * b[i] + (s0 + i * T >= clear_end)], 1);
+                    if (b[i] >= 0) atomicAdd(&hist_r[2 * b[i] + (s0 + i * T >= clear_end)], 1);
             }
             if (bad < nsave) atomicMin(nfin_s, bad);
         }
@@ -516,7 +537,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) dmumu_kernel(DmumuLaunch a)
         if (wis == 0) {
             const int per = (nbk + kWarp - 1) / kWarp, b0 = min(lane * per, nbk), b1 = min(b0 + per, nbk);
             int t = 0;
-            for (int b = b0; b < b1; ++b) t += hist[b];
+            for (int b = b0; b < b1; ++b) t += hist[b] + hist_r[b];
             int incl = t;
 #pragma unroll
             for (int d = 1; d < kWarp; d <<= 1) {
@@ -527,44 +548,55 @@ __global__ void __launch_bounds__(kMaxThreads, 1) dmumu_kernel(DmumuLaunch a)
             for (int b = b0; b < b1; ++b) {
                 const int h = hist[b];
                 cur[b] = run;
-                next[b] = run;
-                run += h;
+                next[b] = run + h;
+                run += h + hist_r[b];
             }
             if (lane == kWarp - 1) cur[nbk] = run;
         }
         slot_barrier(slot, T);
         const int nfin = *nfin_s, total = cur[nbk];
         const bool prefix = total == nfin;  // every finite save comes before the first non-finite one
-        // ---- the list, and the lags each start reaches (the bin again: cheaper
-        // than the registers that would carry it over the barriers)
-        for (int s0 = st; s0 < nsave; s0 += kBatch * T) {
-            MuT v[kBatch];
-            int b[kBatch], at[kBatch];
+        // ---- the list, and the lags each start reaches (beyond kKeep saves per
+        // thread the bin is computed again)
+        {
+            auto reach = [&](int s, int b) {
+                if (!prefix || b >= nb) return;
+                const int k = MODE == SLOT_REP ? (int)ktab[nfin - s] : lags_below(nfin - s);
+                atomicAdd(&hist2[b * (nl + 1) + k], 1u);
+            };
 #pragma unroll
-            for (int i = 0; i < kBatch; ++i) {
-                const int s = s0 + i * T;
-                if constexpr (MODE == SLOT_REP)
-                    v[i] = s < nsave ? *(const MuT*)((const char*)series + 16 * (size_t)s) : MuT(NAN);
-                else
-                    v[i] = s < nsave ? series[s] : MuT(NAN);
+            for (int i = 0; i < kKeep; ++i) {
+                if (i * T >= nsave) break;
+                if (pk[i] == 0xffffffffu || i * T + st >= nsave) continue;
+                const int k = (int)(pk[i] >> 16);
+                list[cur[k] + (int)(pk[i] & 0xffffu)] = (IdxT)(i * T + st);
+                reach(i * T + st, k >> 1);
             }
-            bins_of(v, E, b);
+            for (int s0 = kKeep * T + st; s0 < nsave; s0 += kBatch * T) {
+                MuT v[kBatch];
+                int b[kBatch], at[kBatch];
 #pragma unroll
-            for (int i = 0; i < kBatch; ++i)
-                at[i] = b[i] >= 0 ? atomicAdd(&next[2 * b[i] + (s0 + i * T >= clear_end)], 1) : 0;
+                for (int i = 0; i < kBatch; ++i) {
+                    const int s = s0 + i * T;
+                    if constexpr (MODE == SLOT_REP)
+                        v[i] = s < nsave ? *(const MuT*)((const char*)series + 16 * (size_t)s) : MuT(NAN);
+                    else
+                        v[i] = s < nsave ? series[s] : MuT(NAN);
+                }
+                bins_of(v, E, b);
 #pragma unroll
-            for (int i = 0; i < kBatch; ++i) {
-                const int s = s0 + i * T;
-                if (b[i] < 0) continue;
-                list[at[i]] = (IdxT)s;
-                if (prefix && b[i] < nb) {
-                    const int k = MODE == SLOT_REP ? (int)ktab[nfin - s] : lags_below(nfin - s);
-                    atomicAdd(&hist2[b[i] * (nl + 1) + k], 1u);
+                for (int i = 0; i < kBatch; ++i)
+                    at[i] = b[i] >= 0 ? atomicAdd(&next[2 * b[i] + (s0 + i * T >= clear_end)], 1) : 0;
+#pragma unroll
+                for (int i = 0; i < kBatch; ++i) {
+                    if (b[i] < 0) continue;
+                    list[at[i]] = (IdxT)(s0 + i * T);
+                    reach(s0 + i * T, b[i]);
                 }
             }
         }
         slot_barrier(slot, T);
-        for (int i = st; i < nbk; i += T) hist[i] = 0;
+        for (int i = st; i < 2 * nbk; i += T) hist[i] = 0;
         if (st == 0) *nfin_s = nsave;
         // ---- pairs: shares of the list of equal cost, a flush counted as
         // kFlushCost starts (a bin may straddle two shares; each flushes its
@@ -585,11 +617,11 @@ __global__ void __launch_bounds__(kMaxThreads, 1) dmumu_kernel(DmumuLaunch a)
         const int* lane_lag = s_lane + group * NS * kLagLanes;
         if (prefix)
             dmumu_pairs<MuT, IdxT, NS, MODE, false>(series, list, cur, nfin == nsave, nb, nl, bin0, r0, r1,
-                                                    nfin, off, lane, lane_lag, acc_sd, acc_sd2, cnt_out, tot_sd2,
+                                                    nfin, off, lane, lane_lag, out_sd, out_sd2, out_cnt, tot_sd2,
                                                     tot_c);
         else
             dmumu_pairs<MuT, IdxT, NS, MODE, true>(series, list, cur, false, nb, nl, bin0, r0, r1, nsave,
-                                                   off, lane, lane_lag, acc_sd, acc_sd2, cnt_out, tot_sd2, tot_c);
+                                                   off, lane, lane_lag, out_sd, out_sd2, out_cnt, tot_sd2, tot_c);
         slot_barrier(slot, T);
         // ---- per-particle value: mean dmu^2 over its valid pairs (dmumu:528-537).
         // The next particle's staging may start: what it shares with this (hist,
@@ -625,11 +657,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1) dmumu_kernel(DmumuLaunch a)
     }
     __syncthreads();
     for (int i = threadIdx.x; i < nl * nb; i += blockDim.x) {
-        const int l = i / nb, b = i % nb;  // partials are [lag][bin], the shared sums [bin][lag]
-        a.part_sd[cta * nl * nb + i] = acc_sd[b * nl + l];
-        a.part_sd2[cta * nl * nb + i] = acc_sd2[b * nl + l];
-        const unsigned c = hist2[b * (nl + 1) + s_rank[l] + 1];  // starts that reach more lags than this one's rank
-        if (c) atomicAdd(&cnt_out[i], (unsigned long long)c);
+        const unsigned c = hist2[i / nl * (nl + 1) + s_rank[i % nl] + 1];  // starts that reach more lags than this one's rank
+        if (c) atomicAdd(&out_cnt[i], (unsigned long long)c);
     }
     for (int l = threadIdx.x; l < nl; l += blockDim.x) {
         WelfordPart r{0, 0.0, 0.0, 0.0, 0};
@@ -685,7 +714,7 @@ __global__ void __launch_bounds__(kWarp* kFinRows)
                 sd += ss[r][x];
                 sd2 += ss2[r][x];
             }
-            const int l = t / nb, b = t % nb;
+            const int l = t % nl, b = t / nl;                // partials are [bin][lag]
             const int64_t o = (int64_t)(lag0 + l) * nb + b;  // Julia (n_bins, n_lags)
             counts[o] += (int64_t)c;
             sum_d[o] += sd;
@@ -900,10 +929,9 @@ __global__ void __launch_bounds__(kInjThreads) dmumu_injection_kernel(DmumuInjec
     __syncthreads();
     const int64_t cta = blockIdx.x;
     for (int i = threadIdx.x; i < nl * nb; i += blockDim.x) {
-        const int j = (i % nb) * nl + i / nb;  // partials are [lag][bin], the shared sums [bin][lag]
-        a.part_cnt[cta * nl * nb + i] = acc_cnt[j];
-        a.part_sd[cta * nl * nb + i] = acc_sd[j];
-        a.part_sd2[cta * nl * nb + i] = acc_sd2[j];
+        a.part_cnt[cta * nl * nb + i] = acc_cnt[i];
+        a.part_sd[cta * nl * nb + i] = acc_sd[i];
+        a.part_sd2[cta * nl * nb + i] = acc_sd2[i];
     }
     for (int l = threadIdx.x; l < nl; l += blockDim.x) {
         WelfordPart r{0, 0.0, 0.0, 0.0, 0};
@@ -971,8 +999,8 @@ DmumuShape dmumu_shape(int64_t n, int64_t nsave, int nl, int n_bins, int mu_byte
     // rounds of particles times the time of one, which falls with the warps on
     // it but for a constant part (barriers, the scan); the larger ppc among equals
     double best = 0.0;
-    for (int c = 1; c <= max_ppc && c * h.groups * kWarp <= kMaxThreads; ++c) {
-        const int pt = std::max(1, kMaxThreads / (kWarp * c * h.groups));
+    for (int c = 1; c <= max_ppc && c * h.groups * kWarp <= max_threads(h.ns); ++c) {
+        const int pt = std::max(1, max_threads(h.ns) / (kWarp * c * h.groups));
         const double rounds = (double)((n + (int64_t)c * num_sms - 1) / ((int64_t)c * num_sms));
         const double cost = rounds * (1.0 / pt + 0.02);
         if (best == 0.0 || cost <= best) {
