@@ -640,8 +640,15 @@ int pt_push_run(pt_ctx* ctx, const pt_field* f, double* x1, double* x2, double* 
     // transpose turns each chunk into the rows the callback receives.
     const bool tf = p->precision == PT_PUSH_F32 && p->cache_mode == PT_CACHE_MU && !p->cache_f64 && n > 0;
     const int tf_pitch = 8;
-    // rows per egress chunk: enough steps per launch, bounded staging memory
-    int64_t R = tf ? tf_pitch : std::max<int64_t>(1, (256 + stride - 1) / stride);
+    // Rows per egress chunk: the rows of 64 steps (one launch), so that the rows of
+    // one chunk are handed over while the next chunks run -- a 256-step run in one
+    // chunk pushed first and handed over all its rows after that (65,536
+    // particles, FP64, phase space: 8.7 ms, 6.4 in four chunks) -- with bounded
+    // staging memory.  The sorted FP64 push copies and sorts the state once per
+    // chunk: 256 steps.
+    const bool resort = p->precision == PT_PUSH_F64 && f->storage == PT_FIELD_BRICK_F64 && p->sort_every > 0;
+    const int64_t steps_per_chunk = resort ? 256 : 64;
+    int64_t R = tf ? tf_pitch : std::max<int64_t>(1, (steps_per_chunk + stride - 1) / stride);
     const size_t slot_cap = tf ? (512u << 20) : (256u << 20);
     if (row_bytes > 0) R = std::max<int64_t>(1, std::min<int64_t>(R, (int64_t)(slot_cap / row_bytes)));
     const int64_t chunk_steps = R * stride;
