@@ -284,3 +284,36 @@ def test_batch_launch_shapes_bit_identical(cuda, threads, bps):
     with pytest.raises(PtError, match="threads_per_block"):
         b.set_launch(96, 2)
     b.close()
+
+
+@pytest.mark.parametrize("sizes", [(1, 2560, 255, 256), (257, 1, 1, 3000), (5, 5, 5, 5), (513,)])
+def test_batch_tile_order_bit_identical(cuda, sizes):
+    """The campaigns' tiles are dealt side by side: one tile against many, equal
+    counts, tile remainders, a single campaign, and the table rebuilt after a
+    campaign has left -- every campaign still equals its run alone."""
+    torch = cuda
+    pb = small_problem(n=16, n_particles=10, u_over_c=1e-4, seed=3)
+    fl = FieldLibrary(pb.fields, pb.grid, "brick_f32")
+    g0 = energy_to_gamma(1.0)
+    dt = (2 * math.pi / 64) / reference_Omega0(pb.B0, g0, F.Q_E, F.M_P)
+    cs = [dict(field=fl, state=init_particles(n, pb.grid, 1.0, seed=40 + i), dt=dt, nsteps=97, stride=8)
+          for i, n in enumerate(sizes)]
+    ref = [run_alone(torch, c) for c in cs]
+    b = Batch(sum(sizes) + 64, max_campaigns=8, storage="brick_f32", steps_per_epoch=32, sort=True)
+    caches = [new_cache(torch, c) for c in cs]
+    ids = [b.add(c["field"], c["state"], c["dt"], c["nsteps"], c["stride"], cache=ch, sort_every=1)
+           for c, ch in zip(cs, caches)]
+    b.run(2)
+    gone = len(cs) - 1 if len(cs) > 1 else None
+    if gone is not None:
+        b.remove(ids[gone])
+    b.run(2)
+    for i, (c, cid, ch, (mu_ref, st_ref)) in enumerate(zip(cs, ids, caches, ref)):
+        if i == gone:
+            continue
+        assert b.step(cid) == c["nsteps"]
+        assert np.array_equal(ch.cpu().numpy(), mu_ref, equal_nan=True)
+        st, _ = b.export(cid)
+        for k in st:
+            assert np.array_equal(st[k].cpu().numpy(), st_ref[k]), k
+    b.close()
