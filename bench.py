@@ -61,7 +61,8 @@ def parse():
     ap.add_argument("--energy", type=float, default=10.0)
     ap.add_argument("--storage", default="brick_bf16", choices=["brick_bf16", "brick_bf16x", "brick_f32"])
     ap.add_argument("--sort-every", type=int, default=64, help="re-sort particles by brick every N pushes (0: never)")
-    ap.add_argument("--variant", type=int, default=1, help="push launch shape (pt_push_params.kernel_variant)")
+    ap.add_argument("--variant", type=int, default=0,
+                    help="push launch shape (pt_push_params.kernel_variant; 0: chosen by the library)")
     ap.add_argument("--lag-particles", type=int, default=1_048_576)
     ap.add_argument("--dpp-particles", type=int, default=262_144)
     ap.add_argument("--e2e-gyroperiods", type=int, default=500,
@@ -617,7 +618,7 @@ def run_ours(args, ws, rank, local):
         dpp_s = dms / 2 / 1e3
         dpp = {"value": ws * dpairs / max_over_ranks(dpp_s * 1e3, ws, dev) * 1e3, "unit": "lag-pairs/s",
                "pairs_per_pass": dpairs, "ms_per_pass": dms / 2, "particles": npp, "saves": nsave,
-               "lags": int(len(lags_p)), "estimator": "sliding, |p| recomputed per end in FP64",
+               "lags": int(len(lags_p)), "estimator": "sliding, |p| once per save in FP64",
                "compulsory_bytes_per_pass": 12 * npp * nsave,
                "hbm_frac_of_compulsory": (12 * npp * nsave / dpp_s / 1e9) / peaks["hbm_gbs"],
                "phase_space_push_s": ps_push_s, "phase_space_push_rate": npp * (NSTEPS - 1) / ps_push_s,
@@ -711,7 +712,8 @@ def run_ours(args, ws, rank, local):
 # small case (profiles/dmumu_*.md, profiles/dpp_*.md).  These kernels are
 # bound by instruction issue, whose ceiling is one warp instruction per cycle
 # per SM sub-partition (4 per SM).
-WARP_INST_PER_PAIR = {"dmumu_kernel": 47.59e9 / 49.193e9, "dpp_kernel": 6.663e9 / 12.298e9}
+# D_pp counts its two kernels (pmag_kernel and dpp_kernel).
+WARP_INST_PER_PAIR = {"dmumu_kernel": 21.777e9 / 49.193e9, "dpp_kernel": (2.861e9 + 0.771e9) / 12.298e9}
 
 
 def issue_roofline(kernel: str, pairs_per_s: float, clocks, device) -> dict:
@@ -736,7 +738,7 @@ def issue_roofline(kernel: str, pairs_per_s: float, clocks, device) -> dict:
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one 64-step
 # push_fast_kernel launch of this workload, from a 1-pass ncu capture of the
 # same command; keyed by (storage, grid, particles)
-TRAFFIC = {("brick_bf16", 512, 16_777_216): 6.63e9 + 1.44e9}
+TRAFFIC = {("brick_bf16", 512, 16_777_216): 4.96e9 + 1.48e9}
 
 
 def run_config1(args, rank):
