@@ -134,8 +134,9 @@ namespace pt {
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // Grow-only device scratch owned by the context (slot = independent user).
-// Slots: 0 D_mumu, 1 D_pp, 2 pt_push_run state, 3 particle initialisation,
-// 4 phase-space D_mumu (interleaved B + mu chunk).
+// Slots: 0 D_mumu partials, 1 D_pp partials + |p| chunk, 2 pt_push_run state,
+// 3 particle initialisation, 4 phase-space D_mumu (B source + mu chunk), 5 slots
+// of the sorted FP64 push.
 int scratch_get(pt_ctx* ctx, int slot, size_t bytes, void** out);
 
 // ---------------------------------------------------------------- host I/O
