@@ -129,8 +129,10 @@ int pt_ctx_set_stream(pt_ctx* ctx, void* cuda_stream);
 int pt_ctx_synchronize(pt_ctx* ctx);
 /* Free the buffers a context keeps between calls: device scratch, the pinned
  * host staging and the particle state of pt_push_run (all grow-only, reused
- * by the next call of the same size).  pt_ctx_destroy frees them too.  No
- * reference counterpart (the reference allocates per run). */
+ * by the next call of the same size), and what its memory pool holds after
+ * calls that took memory for their own duration (at most 256 MiB between
+ * calls).  pt_ctx_destroy frees them too.  No reference counterpart (the
+ * reference allocates per run). */
 int pt_ctx_trim(pt_ctx* ctx);
 
 /* Upload a static field library (load_static_fields output,
@@ -190,6 +192,11 @@ typedef struct pt_fast_state pt_fast_state;
 int pt_fast_state_create(pt_ctx* ctx, const pt_field* field, const double* d_x1, const double* d_x2,
                          const double* d_x3, const double* d_p1, const double* d_p2, const double* d_p3,
                          const uint8_t* d_alive, int64_t n, pt_fast_state** out);
+/* Final state at d_x1..d_alive, in particle order, on the context stream.  It
+ * only reads the state: exports of one state on several streams or contexts may
+ * overlap.  From 2,097,152 particles on it takes up to 128 MiB of device memory
+ * for the duration of the call (and so does the first sort, with 4 bytes per
+ * particle more); where that is not to be had it does without, slower. */
 int pt_fast_state_export(pt_ctx* ctx, const pt_fast_state* st, double* d_x1, double* d_x2, double* d_x3,
                          double* d_p1, double* d_p2, double* d_p3, uint8_t* d_alive);
 int pt_fast_state_destroy(pt_fast_state* st);

@@ -55,6 +55,28 @@ int scratch_get(pt_ctx* ctx, int slot, size_t bytes, void** out)
     return PT_OK;
 }
 
+CallMem::CallMem(pt_ctx* ctx, size_t bytes, cudaStream_t s) : s_(s)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(s, &cap);
+    if (e == cudaSuccess && cap != cudaStreamCaptureStatusNone) return;
+    if (e == cudaSuccess && !ctx->pool) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = ctx->device;
+        uint64_t keep = kPoolKeep;
+        e = cudaMemPoolCreate(&ctx->pool, &props);
+        if (e == cudaSuccess) e = cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        else ctx->pool = nullptr;
+    }
+    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&p_, bytes, ctx->pool, s);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        p_ = nullptr;
+    }
+}
+
 namespace {
 
 struct DevBuf {
@@ -427,6 +449,7 @@ int pt_ctx_destroy(pt_ctx* ctx)
     ::pt::DeviceScope device_scope(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     pt_ctx_trim(ctx);
+    if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     delete ctx;
@@ -449,6 +472,7 @@ int pt_ctx_trim(pt_ctx* ctx)
     ctx->pinned.bytes = 0;
     if (ctx->run_fs) pt_fast_state_destroy(ctx->run_fs);
     ctx->run_fs = nullptr;
+    if (ctx->pool) PT_CUDA(cudaMemPoolTrimTo(ctx->pool, 0));
     return PT_OK;
 }
 
@@ -570,8 +594,7 @@ int pt_fast_state_export(pt_ctx* ctx, const pt_fast_state* st, double* d_x1, dou
     PT_DEVICE_SCOPE(ctx->device);
     if (st->n == 0) return PT_OK;
     if (!(d_x1 && d_x2 && d_x3 && d_p1 && d_p2 && d_p3 && d_alive)) return fail(PT_ERR_ARG, "null state");
-    // the state's values are not changed, but its record memory may be allocated
-    return launch_fast_export(const_cast<pt_fast_state*>(st), st->field, d_x1, d_x2, d_x3, d_p1, d_p2, d_p3, d_alive, ctx->stream);
+    return launch_fast_export(ctx, st, st->field, d_x1, d_x2, d_x3, d_p1, d_p2, d_p3, d_alive, ctx->stream);
 }
 
 int pt_fast_state_destroy(pt_fast_state* st)
@@ -588,7 +611,6 @@ int pt_fast_state_destroy(pt_fast_state* st)
     if (st->pid_alt) cudaFree(st->pid_alt);
     if (st->alive_alt) cudaFree(st->alive_alt);
     if (st->sort_tmp) cudaFree(st->sort_tmp);
-    if (st->records) cudaFree(st->records);
     delete st;
     return PT_OK;
 }
@@ -769,7 +791,7 @@ int pt_push_run(pt_ctx* ctx, const pt_field* f, double* x1, double* x2, double* 
     rc = deliver(pend);
     if (rc) return finish(rc);
     if (fs) {
-        rc = launch_fast_export(fs, f, d[0], d[1], d[2], d[3], d[4], d[5], dal, st);
+        rc = launch_fast_export(ctx, fs, f, d[0], d[1], d[2], d[3], d[4], d[5], dal, st);
         if (rc) return finish(rc);
     }
     rc = staged_d2h(segs, stage, stage_chunk, stage_nbuf, st);

@@ -83,6 +83,7 @@ struct pt_ctx {
     cudaStream_t stream = nullptr;      // stream used by *_device calls
     cudaStream_t copy_stream = nullptr; // egress copies in pt_push_run
     pt::ScratchBuf scratch[6];          // reusable device scratch, grown on demand
+    cudaMemPool_t pool = nullptr;       // memory that lives for one call (CallMem), created on first use
     pt::ScratchBuf pinned;              // pinned host staging of pt_push_run, grown on demand
     pt_fast_state* run_fs = nullptr;    // FP32-push state reused by pt_push_run
 };
@@ -123,7 +124,6 @@ struct pt_fast_state {
     const pt_field* field = nullptr; // field the state was created against (grid, units)
     int64_t last_sort = INT64_MIN;   // step of the last brick re-sort
     bool sorted = false;             // the slots have been in brick order since the import
-    void* records = nullptr;         // large states: scatters of a random order go through it (push_fast.cu)
     // scratch for the re-sort
     void* sort_tmp = nullptr;
     size_t sort_tmp_bytes = 0;
@@ -138,6 +138,29 @@ inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 // 3 particle initialisation, 4 phase-space D_mumu (B source + mu chunk), 5 slots
 // of the sorted FP64 push.
 int scratch_get(pt_ctx* ctx, int slot, size_t bytes, void** out);
+
+// Device memory of one call, allocated and freed in the order of the call's
+// stream: calls of one context on several streams never share it, as they would
+// the context's scratch, and giving it back stalls nobody, as cudaFree does.  Null
+// where it is not to be had or the stream is capturing; the caller then takes a
+// path that needs none.  The context's pool holds at most kPoolKeep bytes of it
+// between calls.
+constexpr uint64_t kPoolKeep = 256u << 20;
+class CallMem {
+public:
+    CallMem(pt_ctx* ctx, size_t bytes, cudaStream_t s);
+    ~CallMem()
+    {
+        if (p_) cudaFreeAsync(p_, s_);
+    }
+    CallMem(const CallMem&) = delete;
+    CallMem& operator=(const CallMem&) = delete;
+    void* get() const { return p_; }
+
+private:
+    void* p_ = nullptr;
+    cudaStream_t s_ = nullptr;
+};
 
 // ---------------------------------------------------------------- host I/O
 // Grow-only pinned host buffer of the context.
@@ -365,8 +388,8 @@ int launch_batch_export(BatchStateDev st0, BatchStateDev st1, const BatchCampaig
                         double* p3, uint8_t* alive, int num_sms, cudaStream_t s);
 int launch_fast_import(pt_fast_state* st, const pt_field* f, const double* x1, const double* x2, const double* x3,
                        const double* p1, const double* p2, const double* p3, const uint8_t* alive, cudaStream_t s);
-int launch_fast_export(pt_fast_state* st, const pt_field* f, double* x1, double* x2, double* x3, double* p1,
-                       double* p2, double* p3, uint8_t* alive, cudaStream_t s);
+int launch_fast_export(pt_ctx* ctx, const pt_fast_state* st, const pt_field* f, double* x1, double* x2, double* x3,
+                       double* p1, double* p2, double* p3, uint8_t* alive, cudaStream_t s);
 int fast_sort(pt_ctx* ctx, pt_fast_state* st, const pt_field* f, cudaStream_t s);
 
 int launch_brick_convert(const double* const comps[6], const pt_grid& g, double B_ref, int layout, void* nodes,

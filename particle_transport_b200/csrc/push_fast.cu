@@ -14,6 +14,8 @@
 //   p~' = p+ + eps,   x~ += p~' (c dt/dx) / g'
 // and |p|^2 is advanced in FP64 by the two E kicks only, so with E = 0 the
 // particle energy is conserved to FP64 rounding.
+#include <optional>
+
 #include "pt_internal.cuh"
 
 namespace pt {
@@ -1035,33 +1037,14 @@ int launch_fast_import(pt_fast_state* st, const pt_field* f, const double* x1, c
     return PT_OK;
 }
 
-// The state's own record memory -- kRecordWindow records, then a place per particle
-// -- or null where records do not pay or it is not to be had (the direct scatter
-// needs none).  Allocated on first use, but not inside a stream capture.
-static StateRecord* record_window(pt_fast_state* st, cudaStream_t s)
-{
-    if (st->n < kRecordMin) return nullptr;
-    if (!st->records) {
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-            cudaGetLastError();
-            return nullptr;
-        }
-        const size_t bytes = sizeof(StateRecord) * (size_t)std::min(st->n, kRecordWindow) + sizeof(uint32_t) * st->n;
-        if (cudaMalloc(&st->records, bytes) != cudaSuccess) {
-            cudaGetLastError();
-            st->records = nullptr;
-        }
-    }
-    return (StateRecord*)st->records;
-}
-
-int launch_fast_export(pt_fast_state* st, const pt_field* f, double* x1, double* x2, double* x3,
+int launch_fast_export(pt_ctx* ctx, const pt_fast_state* st, const pt_field* f, double* x1, double* x2, double* x3,
                        double* p1, double* p2, double* p3, uint8_t* alive, cudaStream_t s)
 {
     const pt_grid& g = f->grid;
-    const int sms = st->ctx->num_sms;
-    if (StateRecord* rec = record_window(st, s)) {
+    const int sms = ctx->num_sms;
+    std::optional<CallMem> mem;
+    if (st->n >= kRecordMin) mem.emplace(ctx, sizeof(StateRecord) * (size_t)kRecordWindow, s);
+    if (StateRecord* rec = mem ? (StateRecord*)mem->get() : nullptr) {
         for (int64_t d0 = 0; d0 < st->n; d0 += kRecordWindow) {
             const int64_t c = std::min(kRecordWindow, st->n - d0);
             record_pack_kernel<<<grid_for(st->n, 256, sms), 256, 0, s>>>((const uint32_t*)st->pid, (uint32_t)d0,
@@ -1139,9 +1122,11 @@ int fast_sort(pt_ctx* ctx, pt_fast_state* st, const pt_field* f, cudaStream_t s)
     const unsigned sb = (unsigned)((n + kScatterBlock - 1) / kScatterBlock);
     // a state's first sort finds its particles in no order: 16.7M particles take
     // 4.9 ms scattered directly.  Later ones find them in runs (0.9 ms).
-    StateRecord* rec = st->sorted ? nullptr : record_window(st, s);
-    if (rec) {
-        uint32_t* place = (uint32_t*)(rec + std::min(n, kRecordWindow));
+    std::optional<CallMem> mem;
+    if (!st->sorted && n >= kRecordMin)
+        mem.emplace(ctx, sizeof(StateRecord) * (size_t)kRecordWindow + sizeof(uint32_t) * (size_t)n, s);
+    if (StateRecord* rec = mem ? (StateRecord*)mem->get() : nullptr) {
+        uint32_t* place = (uint32_t*)(rec + kRecordWindow);
         sort_place_kernel<<<sb, kScatterBlock, 0, s>>>(cur, tile_off, n, f->offs, nx, ny, nz, nb, st->x, st->alive,
                                                        place);
         PT_CHECK_LAUNCH("sort_place_kernel");

@@ -395,3 +395,41 @@ def test_large_state_through_records_bit_identical(cuda):
         assert torch.equal(a[k], b[k]), k
         assert torch.equal(a[k][n - 1500:], c[k]), k
     assert torch.equal(al, bl) and torch.equal(al[n - 1500:], cl) and torch.equal(al.cpu(), torch.as_tensor(alive))
+
+
+def test_overlapping_exports_of_one_state(cuda):
+    """An export only reads the state: exports of one large sorted state that overlap on several streams, from one
+    context and from several, all give what a single one gives."""
+    torch = cuda
+    from particle_transport_b200 import _lib
+    n = (1 << 22) + 3
+    pb = small_problem(n=16, n_particles=1000, u_over_c=1e-4, energy_GeV=3.0)
+    i = torch.arange(n, device="cuda", dtype=torch.float64)
+    st = {k: torch.as_tensor(v, device="cuda").repeat(n // 1000 + 1)[:n] * (1.0 + 1e-9 * i)
+          for k, v in pb.state.items()}
+    for k in ("x1", "x2", "x3"):
+        st[k] = torch.remainder(st[k], pb.grid.xmax)
+    alive = torch.ones(n, dtype=torch.uint8, device="cuda")
+    alive[::5] = 0
+    ens = R.FastEnsemble(FieldLibrary(pb.fields, pb.grid, "brick_bf16"), st, alive)
+    ens.sort()
+    want, want_alive = ens.export()
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(4)]
+    ctxs = [_lib.Context(0) for _ in range(2)]
+    outs = [({k: torch.full((n,), -1.0, dtype=torch.float64, device="cuda") for k in R.KEYS},
+             torch.full((n,), 9, dtype=torch.uint8, device="cuda")) for _ in streams]
+    torch.cuda.synchronize()
+    for s, (o, al), ctx in zip(streams, outs, [None, None, *ctxs]):
+        with torch.cuda.stream(s):
+            c = ctx or _lib.torch_context(0)
+            c.use_stream(s)
+            _lib.call("pt_fast_state_export", c.handle, ens.handle, *[_lib.ptr(o[k]) for k in R.KEYS], _lib.ptr(al))
+    torch.cuda.synchronize()
+    for o, al in outs:
+        for k in R.KEYS:
+            assert torch.equal(o[k], want[k]), k
+        assert torch.equal(al, want_alive)
+    for c in ctxs:
+        c.close()
+    ens.close()
