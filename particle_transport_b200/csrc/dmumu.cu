@@ -39,6 +39,7 @@
 #include <math_constants.h>
 
 #include <algorithm>
+#include <cfloat>
 #include <mutex>
 #include <type_traits>
 
@@ -85,9 +86,14 @@ __device__ __forceinline__ void welford_merge(long long& gc, double& gm, double&
 
 // Bin edges at the series' precision.  mu is compared with the stored Float64
 // edges; for a Float32 mu, edge <= mu is the same as (edge rounded up to
-// Float32) <= mu, and mu > edge the same as mu > (edge rounded down).
-__device__ __forceinline__ float edge_up(double e, float) { return __double2float_ru(e); }
-__device__ __forceinline__ double edge_up(double e, double) { return e; }
+// Float32) <= mu, and mu > edge the same as mu > (edge rounded down).  A first edge
+// of -Inf becomes the lowest finite value: the same for every finite mu, and a mu of
+// -Inf, which has no bin, fails the comparison that bins_of makes first.
+__device__ __forceinline__ float edge_up(double e, float)
+{
+    return e == -CUDART_INF ? -FLT_MAX : __double2float_ru(e);
+}
+__device__ __forceinline__ double edge_up(double e, double) { return e == -CUDART_INF ? -DBL_MAX : e; }
 __device__ __forceinline__ float edge_down(double e, float) { return __double2float_rd(e); }
 __device__ __forceinline__ double edge_down(double e, double) { return e; }
 

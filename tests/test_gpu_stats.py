@@ -122,6 +122,22 @@ def test_dmumu_edge_values(cuda, oracle):
         check_dmumu(gpu_dmumu(mu, lags, edges, bin_abs=bin_abs), o)
 
 
+@pytest.mark.parametrize("mode", ["sliding", "injection"])
+@pytest.mark.parametrize("edges", [[-np.inf, -0.5, 0.0, 0.5, np.inf], [-np.inf, 0.25], [-1.0, 0.0, np.inf]])
+def test_dmumu_infinite_edges(cuda, oracle, mode, edges):
+    """Signed bins open to one or both sides: finite values of any size have a bin, NaN and the infinities have
+    none."""
+    vals = np.array([0.0, -0.5, 0.25, 1.0, -1.0, 3e3, -3e3, np.nan, np.inf, -np.inf], np.float32)
+    edges = np.array(edges)
+    mu = np.ascontiguousarray(np.random.default_rng(4).choice(vals[[0, 1, 2, 3, 4, 7, 8, 9]], size=(97, 130)))
+    mu[:, 0] = np.resize(vals, 97)  # the injection estimator's starts
+    lags = np.array([1, 2, 64, 129, 500])
+    o = zero_dmumu(len(lags), len(edges) - 1)
+    oracle.dmumu_accumulate(mu, lags, edges, o, injection=mode == "injection", bin_abs=False)
+    assert all(np.isfinite(o[k]).all() for k in ("sum_d", "sum_d2", "w_mean"))
+    check_dmumu(gpu_dmumu(mu, lags, edges, start_mode=mode, bin_abs=False), o)
+
+
 def test_dmumu_rejects_bad_lags(cuda):
     from particle_transport_b200._lib import PtError
     mu = random_mu_cache(4, 10)
