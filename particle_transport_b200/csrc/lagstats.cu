@@ -106,9 +106,10 @@ __host__ __device__ inline DppFixed dpp_fixed(int sets, int nl, int ppc)
 }
 
 // Starts [s0, s1) against NL lags: p[s + L[k]] - p[s], added to sd[k] and sq[k].
-// TEST: only finite differences count (into cnt).
+// TEST: only finite differences count (into cnt).  Starts are unsigned: a series may
+// hold nearly 2^31 saves, and the loops look a pass past the end.
 template <int NL, bool TEST>
-__device__ __forceinline__ void dpp_rows(const double* __restrict__ p, int s0, int s1, const int (&L)[kDppLags], int lane,
+__device__ __forceinline__ void dpp_rows(const double* __restrict__ p, unsigned s0, unsigned s1, const int (&L)[kDppLags], int lane,
                                          double (&sd)[kDppLags], double (&sq)[kDppLags], int (&cnt)[kDppLags])
 {
     auto pair = [&](double ps, double pe, int k) {
@@ -121,7 +122,7 @@ __device__ __forceinline__ void dpp_rows(const double* __restrict__ p, int s0, i
         sd[k] += d;
         sq[k] = fma(d, d, sq[k]);
     };
-    int s = s0 + lane;
+    unsigned s = s0 + lane;
     for (; s + (kDppUnroll - 1) * kWarp < s1; s += kDppUnroll * kWarp) {
         double ps[kDppUnroll], pe[kDppUnroll][NL];
 #pragma unroll

@@ -400,3 +400,44 @@ def test_phase_space_dmumu_b_sources(cuda, oracle, dtype, mode, b_layout, monkey
                                       g["particle_m2s"], g["pair_sum_squares"], g["pair_counts"], g["dmumu_counts"],
                                       g["dmumu_sum_delta"], g["dmumu_sum_delta2"], start_mode=mode)
     check_dmumu({k: v.cpu().numpy() for k, v in g.items()}, o)
+
+
+@pytest.mark.parametrize("kind", ["dmumu", "dpp"])
+def test_longest_series(cuda, kind):
+    """One particle with the most saves that the entries take, 2^31 - 2: loops over saves and starts end where the
+    series does.  The values are multiples of a power of two, so that every sum is exact."""
+    torch = cuda
+    ns = 2**31 - 2
+    if torch.cuda.mem_get_info()[0] < 80 << 30:
+        pytest.skip("needs 80 GB of device memory")
+    lags = np.array([1, ns - 1, 7, ns - 3])
+    if kind == "dmumu":
+        vals = np.array([0.125, 0.25, 0.5, 0.75, 0.875])
+        mu = torch.as_tensor(vals, dtype=torch.float32, device="cuda").repeat(ns // 5 + 1)[:ns].view(1, ns)
+        acc = S.new_dmumu_accumulators(len(lags), 5, device="cuda")
+        gpu_dmumu(mu, lags, np.linspace(0.0, 1.0, 6), acc=acc)
+        g = {k: v.cpu().numpy() for k, v in acc.items()}
+        del mu
+        for i, L in enumerate(lags):
+            c = (ns - L - np.arange(5) + 4) // 5  # starts of each value that reach the lag
+            d = np.roll(vals, -(L % 5)) - vals
+            assert np.array_equal(g["dmumu_counts"][i], c)
+            assert np.array_equal(g["dmumu_sum_delta"][i], c * d)
+            assert np.array_equal(g["dmumu_sum_delta2"][i], c * d * d)
+            assert g["pair_counts"][i] == ns - L and g["particle_counts"][i] == 1
+            assert g["particle_means"][i] == (c * d * d).sum() / (ns - L)
+    else:
+        vals = np.array([1.0, 2.0, 4.0]) * 2.0**-63
+        mom = torch.zeros((ns, 3, 1), dtype=torch.float32, device="cuda")
+        mom[:, 1, 0] = torch.as_tensor(vals, dtype=torch.float32, device="cuda").repeat(ns // 3)
+        acc = S.new_dpp_accumulators(len(lags), device="cuda")
+        S.process_momenta_chunk_dpp(mom, lags, 1.0, acc["counts"], acc["sum_delta_p"], acc["sum_delta_p2"],
+                                    acc["sum_delta_p_norm"], acc["sum_delta_p_norm2"])
+        g = {k: v.cpu().numpy() for k, v in acc.items()}
+        del mom
+        for i, L in enumerate(lags):
+            c = (ns - L - np.arange(3) + 2) // 3
+            d = np.roll(vals, -(L % 3)) - vals
+            assert g["counts"][i] == ns - L
+            assert g["sum_delta_p"][i] == (c * d).sum() and g["sum_delta_p2"][i] == (c * d * d).sum()
+    torch.cuda.empty_cache()
