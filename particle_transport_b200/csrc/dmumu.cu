@@ -1122,7 +1122,7 @@ int run_dmumu_t(const PartSource& src, const DmumuArgs& a, const MuT* mu, int64_
             threads = h.ppc * h.groups * h.parts * kWarp;
             blocks = (a.n + h.ppc - 1) / h.ppc;
         }
-        PT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PT_CUDA(allow_smem(kfn, smem));
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, threads, smem);
         blocks = std::min<int64_t>(blocks, (int64_t)ctx->num_sms * std::max(1, per_sm));
         if (src.fixed) {

@@ -630,7 +630,7 @@ int run_dpp(pt_ctx* ctx, const DppArgs& a, cudaStream_t s)
             ++ppc;
         const size_t smem = smem_slots ? need(ppc) : dpp_fixed(L.sets, nl, ppc).series;
         void* kfn = smem_slots ? (void*)dpp_kernel<true> : (void*)dpp_kernel<false>;
-        PT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PT_CUDA(allow_smem(kfn, smem));
         int per_sm = 1;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, kDppThreads, smem);
         const int64_t ctas = (int64_t)ctx->num_sms * std::max(1, per_sm);
@@ -682,8 +682,7 @@ int launch_energy_histogram(const float* mom, int64_t chunk, int64_t nsave, cons
     if (total <= 0) return PT_OK;
     const size_t smem = sizeof(unsigned long long) * (size_t)n_snap * n_hist;
     if (smem > 160 * 1024) return fail(PT_ERR_ARG, "n_snap * n_hist too large for the on-chip histogram");
-    if (smem > 48 * 1024)
-        PT_CUDA(cudaFuncSetAttribute(energy_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) PT_CUDA(allow_smem((const void*)energy_hist_kernel, smem));
     const double log_emin = log(e_min);
     const double inv_dlog = (double)n_hist / (log(e_max) - log_emin);
     const int blocks = (int)std::min<int64_t>((total + 255) / 256, 148 * 4);

@@ -179,6 +179,26 @@ int staged_d2h(const std::vector<HostSeg>& segs, char* stage, size_t chunk, int 
 int64_t count_nonzero(const uint8_t* v, int64_t n);
 
 // ---------------------------------------------------------------- launches
+// Let a kernel launch with `bytes` of dynamic shared memory on the current device.
+// The limit belongs to the kernel on the device, not to a launch, and contexts of
+// several threads share it: every call sets it to all that the kernel can have, so
+// that none lowers it between another's limit and its launch.  own: the kernel has
+// static shared memory beside it (a query of some microseconds).
+inline cudaError_t allow_smem(const void* kfn, size_t bytes, bool own = false)
+{
+    int dev = 0, most = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess && own) {
+        cudaFuncAttributes at{};
+        e = cudaFuncGetAttributes(&at, kfn);
+        most -= (int)at.sharedSizeBytes;
+    }
+    if (e != cudaSuccess) return e;
+    if (bytes > (size_t)most) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
 // Threads per block of a push with one block per SM, at most `most`: the fewest
 // whole warps that take n particles in as many passes over the chip.  (The time of
 // a pass goes with the warps of the fullest scheduler, so rounding up to a warp per

@@ -274,8 +274,7 @@ int launch_push_exact_brick(const PushArgsExactBrick& a, cudaStream_t s)
     const int threads = spread_threads(a.n, kExactThreads);
     const int64_t blocks = (a.n + threads - 1) / threads;
     const size_t smem = a.morton ? 0 : sizeof(uint32_t) * (size_t)(a.g.nx + a.g.ny + a.g.nz);
-    if (smem > 48 * 1024)
-        PT_CUDA(cudaFuncSetAttribute(push_exact_brick_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) PT_CUDA(allow_smem((const void*)push_exact_brick_kernel, smem));
     push_exact_brick_kernel<<<(unsigned)blocks, threads, smem, s>>>(a);
     PT_CHECK_LAUNCH("push_exact_brick_kernel");
     return PT_OK;

@@ -862,7 +862,7 @@ int launch_push_fast_shape(const PushArgsFast& a, cudaStream_t s, int cap_per_sm
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     auto kfn = push_fast_kernel<LAYOUT, BLOCK, MINB, TEXC>;
     if (threads <= 0) threads = BLOCK;
-    if (smem > 48 * 1024) PT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) PT_CUDA(allow_smem((const void*)kfn, smem));
     if (cap_per_sm != 1) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, threads, smem);
     per_sm = std::max(per_sm, 1);
     if (cap_per_sm > 0) per_sm = std::min(per_sm, cap_per_sm);
@@ -1472,7 +1472,7 @@ int launch_push_batch(const BatchLaunch& L, cudaStream_t s)
     void* kfn = L.threads == 64 ? push_batch_fn<64>(L.layout)
                 : (L.threads == 128 ? push_batch_fn<128>(L.layout) : push_batch_fn<kBatchTile>(L.layout));
     const int threads = L.threads == 64 || L.threads == 128 ? L.threads : kBatchTile;
-    if (smem > 48 * 1024) PT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) PT_CUDA(allow_smem(kfn, smem, true));
     BatchLaunch arg = L;
     void* args[] = {&arg};
     PT_CUDA(cudaLaunchKernel(kfn, dim3(L.grid), dim3(threads), args, smem, s));

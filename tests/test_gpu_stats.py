@@ -441,3 +441,52 @@ def test_longest_series(cuda, kind):
             assert g["counts"][i] == ns - L
             assert g["sum_delta_p"][i] == (c * d).sum() and g["sum_delta_p2"][i] == (c * d * d).sum()
     torch.cuda.empty_cache()
+
+
+def test_calls_of_several_threads(cuda):
+    """Threads, each with its own context, make calls of the same kernels that need different amounts of shared
+    memory: every call launches, and the sums are those of the calls alone."""
+    torch = cuda
+    import threading
+    from particle_transport_b200 import _lib
+    lags = torch.as_tensor(np.array([1, 2, 5, 9, 17, 30]), device="cuda")
+    edges = torch.linspace(0.0, 1.0, 11, dtype=torch.float64, device="cuda")
+    ins = [(torch.as_tensor(random_mu_cache(20, ns, seed=ns), device="cuda"), torch.ones((ns, 3, 4), device="cuda"))
+           for ns in (64, 3001, 11000)]
+
+    def calls(ctx, mu, mom, reps):
+        a, b = S.new_dmumu_accumulators(6, 10, device="cuda"), S.new_dpp_accumulators(6, device="cuda")
+        keys = ("dmumu_counts", "dmumu_sum_delta", "dmumu_sum_delta2", "particle_counts", "particle_means",
+                "particle_m2s", "pair_sum_squares", "pair_counts")
+        args = [_lib.ptr(mu), *mu.shape, mu.shape[1], 1, _lib.ptr(lags), 6, _lib.ptr(edges), 10, 0, 1,
+                *[_lib.ptr(a[k]) for k in keys]]
+        dpp = [_lib.ptr(mom), 4, mu.shape[1], _lib.ptr(lags), 6, 1.0,
+               *[_lib.ptr(b[k]) for k in ("counts", "sum_delta_p", "sum_delta_p2", "sum_delta_p_norm",
+                                          "sum_delta_p_norm2")]]
+        torch.cuda.synchronize()
+        for _ in range(reps):
+            _lib.call("pt_dmumu_accumulate_device", ctx.handle, *args)
+            _lib.call("pt_dpp_accumulate_device", ctx.handle, *dpp)
+        ctx.synchronize()
+        return torch.cat([a["dmumu_counts"].flatten(), a["pair_counts"], b["counts"]])
+
+    ctxs = [_lib.Context(0) for _ in ins]
+    want = [calls(c, *i, 1) for c, i in zip(ctxs, ins)]
+    got, errors = [None] * len(ins), []
+
+    def work(i):
+        try:
+            got[i] = calls(ctxs[i], *ins[i], 3000)
+        except Exception as e:
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(ins))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors[0]
+    for g, w in zip(got, want):
+        assert torch.equal(g, 3000 * w)
+    for c in ctxs:
+        c.close()
