@@ -15,6 +15,7 @@
 #include "pt_internal.cuh"
 
 #include <algorithm>
+#include <optional>
 
 namespace pt {
 namespace {
@@ -635,15 +636,27 @@ int run_dpp(pt_ctx* ctx, const DppArgs& a, cudaStream_t s)
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, kDppThreads, smem);
         const int64_t ctas = (int64_t)ctx->num_sms * std::max(1, per_sm);
         const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((a.chunk + ppc - 1) / ppc, ctas));
-        // |p| chunks: whole rounds of the CTAs, as many as 128 MB hold
+        // |p| chunks: whole rounds of the CTAs, as many as 128 MB hold.  The context's
+        // scratch holds the partials and at least one series, 16 MB in all for series
+        // below that, so that it does not grow from call to call (its regrowth stalls
+        // the device).  What does not fit there is memory of this call, or, where that
+        // is not to be had (a nearly full device, a stream capture), more launches on
+        // what the scratch holds.
         const int64_t round = (int64_t)grid * ppc;
         const int64_t rounds = std::max<int64_t>(1, (int64_t)(((size_t)128 << 20) / series) / round);
-        const int64_t step = std::min<int64_t>(a.chunk, round * rounds);
+        int64_t step = std::min<int64_t>(a.chunk, round * rounds);
         const size_t part_bytes = (sizeof(DppPart) * (size_t)grid * nl + 255) & ~(size_t)255;
         void* scratch = nullptr;
-        int rc = scratch_get(ctx, 1, part_bytes + (size_t)step * series, &scratch);
+        int rc = scratch_get(ctx, 1, part_bytes + series, &scratch);
         if (rc) return rc;
         double* pmag = (double*)((char*)scratch + part_bytes);
+        const int64_t held = (int64_t)((ctx->scratch[1].bytes - part_bytes) / series);
+        std::optional<CallMem> mem;
+        if (held < step) {
+            mem.emplace(ctx, (size_t)step * series, s);
+            if (mem->get()) pmag = (double*)mem->get();
+            else step = held >= round ? held / round * round : held;
+        }
         L.pmag = pmag; L.nsave = a.nsave; L.pitch = pitch; L.lags = a.lags + lag0; L.nl = nl;
         L.ppc = ppc;
         L.part = (DppPart*)scratch;

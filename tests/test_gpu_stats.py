@@ -490,3 +490,54 @@ def test_calls_of_several_threads(cuda):
         assert torch.equal(g, 3000 * w)
     for c in ctxs:
         c.close()
+
+
+def test_dpp_on_a_full_device(cuda):
+    """D_pp with less free memory than its |p| chunks would take, and inside a stream capture: the same sums from
+    smaller chunks."""
+    torch = cuda
+    from particle_transport_b200 import _lib
+    n, ns = 20000, 1001
+    g = torch.Generator(device="cuda").manual_seed(5)
+    mom = torch.randn((ns, 3, n), generator=g, device="cuda")
+    mom[500:, :, ::3] = float("nan")
+    lags = torch.as_tensor(log_spaced_lag_steps(ns - 1, 12), device="cuda")
+    nl = len(lags)
+    keys = ("counts", "sum_delta_p", "sum_delta_p2", "sum_delta_p_norm", "sum_delta_p_norm2")
+    accs = [S.new_dpp_accumulators(nl, device="cuda") for _ in range(3)]
+
+    def call(ctx, acc, m=n):
+        _lib.call("pt_dpp_accumulate_device", ctx.handle, _lib.ptr(mom), m, ns, _lib.ptr(lags), nl, 2.0,
+                  *[_lib.ptr(acc[k]) for k in keys])
+
+    call(_lib.torch_context(0), accs[0])
+    ctx = _lib.Context(0)
+    ctx.use_stream(torch.cuda.current_stream())
+    call(ctx, S.new_dpp_accumulators(nl, device="cuda"), 7)  # what the context keeps between calls is there
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    held = []
+    while torch.cuda.mem_get_info()[0] > 96 << 20:
+        held.append(torch.empty(torch.cuda.mem_get_info()[0] - (64 << 20), dtype=torch.uint8, device="cuda"))
+    call(ctx, accs[1])
+    torch.cuda.synchronize()
+    del held
+    torch.cuda.empty_cache()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ctx.use_stream(torch.cuda.current_stream())
+        call(ctx, accs[2])
+    graph.replay()
+    torch.cuda.synchronize()
+    ctx.use_stream(None)
+    want = {k: v.cpu().numpy() for k, v in accs[0].items()}
+    for acc in accs[1:]:
+        got = {k: v.cpu().numpy() for k, v in acc.items()}
+        assert np.array_equal(got["counts"], want["counts"])
+        assert close(got["sum_delta_p2"], want["sum_delta_p2"]) and close(got["sum_delta_p_norm2"],
+                                                                         want["sum_delta_p_norm2"])
+        scale = np.sqrt(np.maximum(want["counts"], 1) * want["sum_delta_p2"])
+        assert close(got["sum_delta_p"], want["sum_delta_p"], scale=scale)
+        assert close(got["sum_delta_p_norm"], want["sum_delta_p_norm"], scale=scale)
+    del graph
+    ctx.close()
