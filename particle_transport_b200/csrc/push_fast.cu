@@ -1042,8 +1042,11 @@ int launch_fast_export(pt_ctx* ctx, const pt_fast_state* st, const pt_field* f, 
 {
     const pt_grid& g = f->grid;
     const int sms = ctx->num_sms;
+    // slots that were never sorted are in id order: the direct export writes them
+    // coalesced, and records would only move them twice more (16.7M particles:
+    // 0.27 ms direct, 0.78 through records; sorted: 4.6 direct, 0.90)
     std::optional<CallMem> mem;
-    if (st->n >= kRecordMin) mem.emplace(ctx, sizeof(StateRecord) * (size_t)kRecordWindow, s);
+    if (st->sorted && st->n >= kRecordMin) mem.emplace(ctx, sizeof(StateRecord) * (size_t)kRecordWindow, s);
     if (StateRecord* rec = mem ? (StateRecord*)mem->get() : nullptr) {
         for (int64_t d0 = 0; d0 < st->n; d0 += kRecordWindow) {
             const int64_t c = std::min(kRecordWindow, st->n - d0);

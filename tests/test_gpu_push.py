@@ -433,3 +433,38 @@ def test_overlapping_exports_of_one_state(cuda):
     for c in ctxs:
         c.close()
     ens.close()
+
+
+def test_export_of_unsorted_slots_needs_no_memory(cuda):
+    """Slots that were never sorted are in id order: a large state's export writes them as they lie, without records
+    in device memory, and a sorted state's gives the same."""
+    torch = cuda
+    from particle_transport_b200 import _lib
+    n = (1 << 21) + 5
+    pb = small_problem(n=16, n_particles=1000, u_over_c=1e-4, energy_GeV=3.0)
+    st = {k: torch.as_tensor(np.resize(v, n), device="cuda") for k, v in pb.state.items()}
+    alive = torch.ones(n, dtype=torch.uint8, device="cuda")
+    alive[::3] = 0
+    ens = R.FastEnsemble(FieldLibrary(pb.fields, pb.grid, "brick_bf16"), st, alive)
+    out = {k: torch.empty(n, dtype=torch.float64, device="cuda") for k in R.KEYS}
+    al = torch.empty(n, dtype=torch.uint8, device="cuda")
+    ctx = _lib.Context(0)
+
+    def export():
+        _lib.call("pt_fast_state_export", ctx.handle, ens.handle, *[_lib.ptr(out[k]) for k in R.KEYS], _lib.ptr(al))
+        ctx.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    assert export() == free
+    ref = {k: v.clone() for k, v in out.items()}
+    assert torch.equal(al, alive)
+    ens.sort()
+    torch.cuda.synchronize()
+    export()
+    for k in R.KEYS:
+        assert torch.equal(out[k], ref[k]), k
+    assert torch.equal(al, alive)
+    ctx.close()
+    ens.close()
