@@ -195,9 +195,9 @@ int pt_fast_state_create(pt_ctx* ctx, const pt_field* field, const double* d_x1,
 /* Final state at d_x1..d_alive, in particle order, on the context stream.  It
  * only reads the state: exports of one state on several streams or contexts may
  * overlap.  From 2,097,152 particles on the export of a state that has been
- * sorted takes 128 MiB of device memory for the duration of the call (and so does
- * the first sort, with 4 bytes per particle more); where that is not to be had it
- * does without, slower. */
+ * sorted takes 128 MiB of device memory, or a byte per particle where that is
+ * more, for the duration of the call (and so does the first sort, with 4 bytes per
+ * particle more); where that is not to be had it does without, slower. */
 int pt_fast_state_export(pt_ctx* ctx, const pt_fast_state* st, double* d_x1, double* d_x2, double* d_x3,
                          double* d_p1, double* d_p2, double* d_p3, uint8_t* d_alive);
 int pt_fast_state_destroy(pt_fast_state* st);

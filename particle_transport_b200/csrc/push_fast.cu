@@ -428,8 +428,10 @@ __global__ void fast_export_kernel(const double* __restrict__ xs, const float* _
 // arrays coalesced.  Scattered directly, each of the nine values costs a 32-byte
 // sector that DRAM reads and writes back: exporting 16.7M particles took 4.7 ms,
 // with records 0.9.  The records hold a window of kRecordWindow places, so that the
-// memory is bounded; each window's pack reads all places.  Below kRecordMin
-// particles the arrays of the direct scatter stay in L2, where its sectors merge.
+// memory is bounded; each window's pack reads all places, so there are at most
+// kRecordWindows of them: beyond 134M particles the window grows with the count (a
+// byte of memory per particle).  Below kRecordMin particles the arrays of the direct
+// scatter stay in L2, where its sectors merge.
 struct alignas(32) StateRecord {
     double x[3], p2;
     float p[3];
@@ -439,7 +441,12 @@ struct alignas(32) StateRecord {
 };
 static_assert(sizeof(StateRecord) == 64, "two sectors");
 constexpr int64_t kRecordWindow = 2 << 20;  // 128 MB
+constexpr int64_t kRecordWindows = 64;
 constexpr int64_t kRecordMin = 1 << 21;
+inline int64_t record_window(int64_t n)
+{
+    return std::max(kRecordWindow, (n + kRecordWindows - 1) / kRecordWindows);
+}
 
 // 32-byte store (sm_100 256-bit vector store; the address is 32-byte aligned)
 __device__ __forceinline__ void stg256(void* p, const uint32_t w[8])
@@ -1046,10 +1053,11 @@ int launch_fast_export(pt_ctx* ctx, const pt_fast_state* st, const pt_field* f, 
     // coalesced, and records would only move them twice more (16.7M particles:
     // 0.27 ms direct, 0.78 through records; sorted: 4.6 direct, 0.90)
     std::optional<CallMem> mem;
-    if (st->sorted && st->n >= kRecordMin) mem.emplace(ctx, sizeof(StateRecord) * (size_t)kRecordWindow, s);
+    const int64_t window = record_window(st->n);
+    if (st->sorted && st->n >= kRecordMin) mem.emplace(ctx, sizeof(StateRecord) * (size_t)window, s);
     if (StateRecord* rec = mem ? (StateRecord*)mem->get() : nullptr) {
-        for (int64_t d0 = 0; d0 < st->n; d0 += kRecordWindow) {
-            const int64_t c = std::min(kRecordWindow, st->n - d0);
+        for (int64_t d0 = 0; d0 < st->n; d0 += window) {
+            const int64_t c = std::min(window, st->n - d0);
             record_pack_kernel<<<grid_for(st->n, 256, sms), 256, 0, s>>>((const uint32_t*)st->pid, (uint32_t)d0,
                                                                          (uint32_t)c, st->n, st->x, st->p, st->p2,
                                                                          st->pid, st->alive, rec);
@@ -1126,15 +1134,16 @@ int fast_sort(pt_ctx* ctx, pt_fast_state* st, const pt_field* f, cudaStream_t s)
     // a state's first sort finds its particles in no order: 16.7M particles take
     // 4.9 ms scattered directly.  Later ones find them in runs (0.9 ms).
     std::optional<CallMem> mem;
+    const int64_t window = record_window(n);
     if (!st->sorted && n >= kRecordMin)
-        mem.emplace(ctx, sizeof(StateRecord) * (size_t)kRecordWindow + sizeof(uint32_t) * (size_t)n, s);
+        mem.emplace(ctx, sizeof(StateRecord) * (size_t)window + sizeof(uint32_t) * (size_t)n, s);
     if (StateRecord* rec = mem ? (StateRecord*)mem->get() : nullptr) {
-        uint32_t* place = (uint32_t*)(rec + kRecordWindow);
+        uint32_t* place = (uint32_t*)(rec + window);
         sort_place_kernel<<<sb, kScatterBlock, 0, s>>>(cur, tile_off, n, f->offs, nx, ny, nz, nb, st->x, st->alive,
                                                        place);
         PT_CHECK_LAUNCH("sort_place_kernel");
-        for (int64_t d0 = 0; d0 < n; d0 += kRecordWindow) {
-            const int64_t c = std::min(kRecordWindow, n - d0);
+        for (int64_t d0 = 0; d0 < n; d0 += window) {
+            const int64_t c = std::min(window, n - d0);
             record_pack_kernel<<<grid_for(n, 256, ctx->num_sms), 256, 0, s>>>(place, (uint32_t)d0, (uint32_t)c, n,
                                                                               st->x, st->p, st->p2, st->pid, st->alive,
                                                                               rec);
