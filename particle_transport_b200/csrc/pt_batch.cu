@@ -32,6 +32,7 @@ struct pt_batch {
     uint32_t* hist = nullptr;
     uint32_t* cursor = nullptr;
     int64_t hist_cap = 0;
+    int64_t l2_bytes = 0;
     int64_t* d_m = nullptr;
     int smem_words = 1;
     std::vector<std::pair<int64_t, int64_t>> free_ranges;  // (start, length), sorted
@@ -91,26 +92,66 @@ void drop_graphs(pt_batch* b)
 
 int64_t campaign_tiles(const BatchCampaignDev& C) { return (C.n + kBatchTile - 1) / kBatchTile; }
 
-// The tile table: the campaigns side by side, each at the same fraction of its
-// slots.  A sorted campaign sweeps its field in brick order, so campaigns that
-// share a field then read a brick at about the same time, and one passage of the
-// field through L2 serves all of them (one campaign after another, six campaigns
-// on a 537 MB field read it from DRAM six times an epoch: 5.3 of 6.5 TB/s); and
-// tiles that wait for DRAM run beside tiles that do not.  Tile k of T goes to
-// bucket (2 k + 1) most / (2 T) of `most`, so a bucket holds at most one tile of
-// a campaign; a counting sort over the buckets, linear in the tiles.
-void interleave_tiles(pt_batch* b, int64_t total, int64_t most)
+// The tile table: one field after another, and the campaigns of a large field side by
+// side, each at the same fraction of its slots.  A sorted campaign sweeps its field in
+// brick order, so campaigns dealt side by side read a brick at about the same time, and
+// one passage of the field through L2 serves all of them.  Campaigns of different
+// fields share nothing: side by side they divide L2 among them and load each other's
+// constants and offset tables at nearly every tile; and a field that L2 holds, or
+// nearly, is not read again anyway.  So a field is dealt when it takes more than twice
+// L2 (252 MB).  Batches run to their end, one campaign after another / dealt: six
+// campaigns on one field of 32-byte nodes, 128^3 45.9 / 46.9 ms, 176^3 (174 MB) 49.4 /
+// 50.0, 192^3 (226 MB) 52.0 / 51.1 and with larger campaigns 98.8 / 100.9, 208^3 (288
+// MB) 54.7 / 51.7, 256^3 93.9 / 88.3; of 16-byte nodes, 192^3 40.7 / 42.0, 256^3 (268
+// MB) 43.7 / 42.5, 320^3 49.2 / 46.8.  Twelve campaigns on four fields of 256^3: 188.0
+// one after another, 195.3 all side by side, 174.9 side by side per field.
+//
+// In a dealt field, tile k of a campaign's T goes to bucket (2 k + 1) most / (2 T) of
+// the `most` tiles of the field's largest campaign, so a bucket holds at most one tile
+// of a campaign; a counting sort over the buckets, linear in the tiles.
+void deal_tiles(pt_batch* b)
 {
     std::vector<BatchTile>& tiles = b->tile_scratch;
     std::vector<int32_t>& first = b->bucket_scratch;
+    struct Group {  // the running campaigns of a field
+        const pt_field* field;
+        bool dealt;
+        int64_t buckets, base;  // tiles of the largest campaign if dealt, of all otherwise; first bucket
+    };
+    struct Place {
+        int group = -1;
+        int64_t offset = 0;  // first bucket in the group
+    };
+    std::vector<Group> groups;  // in the order of their first campaigns
+    std::vector<Place> place((size_t)b->max_camps);
+    int64_t total = 0, buckets = 0;
+    for (int c = 0; c < b->max_camps; ++c) {
+        const BatchCampaignDev& C = b->h_camps[c];
+        if (!C.active || !C.running) continue;
+        const pt_field* field = b->fields[c];
+        size_t f = 0;
+        while (f < groups.size() && groups[f].field != field) ++f;
+        if (f == groups.size()) groups.push_back(Group{field, field->bytes > 2 * b->l2_bytes, 0, 0});
+        Group& G = groups[f];
+        const int64_t T = campaign_tiles(C);
+        place[(size_t)c] = Place{(int)f, G.dealt ? 0 : G.buckets};
+        G.buckets = G.dealt ? std::max(G.buckets, T) : G.buckets + T;
+        total += T;
+    }
+    for (Group& G : groups) {
+        G.base = buckets;
+        buckets += G.buckets;
+    }
     tiles.resize((size_t)total);
-    first.assign((size_t)most + 1, 0);
+    first.assign((size_t)buckets + 1, 0);
     auto each = [&](auto&& fn) {
         for (int c = 0; c < b->max_camps; ++c) {
+            const Place& at = place[(size_t)c];
+            if (at.group < 0) continue;
             const BatchCampaignDev& C = b->h_camps[c];
-            if (!C.active || !C.running) continue;
-            const int64_t T = campaign_tiles(C);
-            for (int64_t k = 0; k < T; ++k) fn(c, C, k, (2 * k + 1) * most / (2 * T));
+            const Group& G = groups[(size_t)at.group];
+            const int64_t T = campaign_tiles(C), most = G.dealt ? G.buckets : T, base = G.base + at.offset;
+            for (int64_t k = 0; k < T; ++k) fn(c, C, k, base + (2 * k + 1) * most / (2 * T));
         }
     };
     each([&](int, const BatchCampaignDev&, int64_t, int64_t bucket) { ++first[(size_t)bucket + 1]; });
@@ -133,16 +174,13 @@ int rebuild_tables(pt_batch* b, int fresh)
 {
     int64_t key = 0;
     std::vector<BatchTile>& tiles = b->tile_scratch;
-    int64_t total = 0, most = 0;  // tiles of all running campaigns, of the largest
     for (int c = 0; c < b->max_camps; ++c) {
         BatchCampaignDev& C = b->h_camps[c];
         if (!C.active || !C.running) continue;
         C.key_base = key;
         key += C.n_bricks + 1;
-        total += campaign_tiles(C);
-        most = std::max(most, campaign_tiles(C));
     }
-    interleave_tiles(b, total, most);
+    deal_tiles(b);
     if (key > UINT32_MAX) return fail(PT_ERR_ARG, "too many sort buckets in the batch");
     if (key > b->hist_cap) {
         const int64_t want = std::max<int64_t>(key, 2 * b->hist_cap);
@@ -273,6 +311,9 @@ int pt_batch_create(pt_ctx* ctx, int64_t capacity, int max_campaigns, int storag
     b->sort = sort ? 1 : 0;
     b->h_camps.assign(max_campaigns, BatchCampaignDev{});
     b->fields.assign(max_campaigns, nullptr);
+    int l2 = 0;
+    cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, ctx->device);
+    b->l2_bytes = l2;
     b->free_ranges.push_back({0, capacity});
     int rc = alloc_state(b->buf[0], capacity);
     if (!rc && b->sort) rc = alloc_state(b->buf[1], capacity);

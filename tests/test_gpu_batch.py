@@ -317,3 +317,52 @@ def test_batch_tile_order_bit_identical(cuda, sizes):
         for k in st:
             assert np.array_equal(st[k].cpu().numpy(), st_ref[k]), k
     b.close()
+
+
+def _big_library(torch):
+    """A field of more than twice the L2 cache, 256^3 FP32 bricks of random values: its campaigns are dealt side by
+    side."""
+    g = torch.Generator(device="cuda").manual_seed(9)
+    fields = [torch.randn((256, 256, 256), generator=g, device="cuda", dtype=torch.float64) * s + m
+              for s, m in ((5e-11, 0.0), (5e-11, 0.0), (5e-11, 1e-10), (3e4, 0.0), (3e4, 0.0), (3e4, 0.0))]
+    grid = F.build_uniform_grid(255 * F.gyroradius_m(1.0, 1e-10), 256, 256, 256)
+    return FieldLibrary(fields, grid, "brick_f32", B_ref_T=1e-10)
+
+
+@pytest.mark.parametrize("sizes", [(1, 2560, 255, 256), (257, 1, 1, 3000), (5, 5, 5, 5)])
+def test_batch_tile_order_over_fields(cuda, sizes):
+    """Campaigns over fields of both tile orders in one batch -- dealt side by side over a large field, one after
+    another over small ones -- whose node offsets are computed (256^3, 16^3) or read from tables that change hands
+    between the tiles (two of 20^3, one of 20 x 12 x 33): every campaign equals its run alone, also after one has
+    left."""
+    torch = cuda
+    libs = [_big_library(torch)]
+    for n, seed in ((20, 3), (16, 4), (20, 5)):
+        pb = small_problem(n=n, n_particles=4, u_over_c=1e-4, seed=seed)
+        libs.append(FieldLibrary(pb.fields, pb.grid, "brick_f32"))
+    pb = small_problem(n=36, n_particles=4, u_over_c=1e-4, seed=6)
+    grid = F.UniformGrid(20, 12, 33, 0.0, 0.0, 0.0, 19 * pb.grid.dx, 11 * pb.grid.dy, 32 * pb.grid.dz, pb.grid.dx,
+                         pb.grid.dy, pb.grid.dz)
+    libs.append(FieldLibrary([np.ascontiguousarray(f[:33, :12, :20]) for f in pb.fields], grid, "brick_f32"))
+    dt = (2 * math.pi / 64) / reference_Omega0(1e-10, energy_to_gamma(1.0), F.Q_E, F.M_P)
+    cs = [dict(field=fl, state=init_particles(n, fl.grid, 1.0, seed=40 + 7 * j + i), dt=dt, nsteps=97, stride=8)
+          for i, n in enumerate(sizes) for j, fl in enumerate(libs)]
+    ref = [run_alone(torch, c) for c in cs]
+    b = Batch(sum(len(c["state"]["x1"]) for c in cs) + 64, max_campaigns=32, storage="brick_f32", steps_per_epoch=32,
+              sort=True)
+    caches = [new_cache(torch, c) for c in cs]
+    ids = [b.add(c["field"], c["state"], c["dt"], c["nsteps"], c["stride"], cache=ch, sort_every=1)
+           for c, ch in zip(cs, caches)]
+    b.run(2)
+    gone = len(cs) - 4  # a campaign of a table field
+    b.remove(ids[gone])
+    b.run(2)
+    for i, (c, cid, ch, (mu_ref, st_ref)) in enumerate(zip(cs, ids, caches, ref)):
+        if i == gone:
+            continue
+        assert b.step(cid) == c["nsteps"]
+        assert np.array_equal(ch.cpu().numpy(), mu_ref, equal_nan=True)
+        st, _ = b.export(cid)
+        for k in st:
+            assert np.array_equal(st[k].cpu().numpy(), st_ref[k]), k
+    b.close()
