@@ -468,3 +468,41 @@ def test_export_of_unsorted_slots_needs_no_memory(cuda):
     assert torch.equal(al, alive)
     ctx.close()
     ens.close()
+
+
+def _table_problem(shape, n_particles):
+    """A grid whose node offsets the push reads from tables (not a power-of-two cube of bricks), cut out of a
+    turbulent cube."""
+    from particle_transport_b200 import fields as F
+    from particle_transport_b200.particles import init_particles
+    nx, ny, nz = shape
+    pb = small_problem(n=max(shape), n_particles=1, u_over_c=1e-4)
+    g = pb.grid
+    pb.fields = [np.ascontiguousarray(f[:nz, :ny, :nx]) for f in pb.fields]
+    pb.grid = F.UniformGrid(nx, ny, nz, 0.0, 0.0, 0.0, (nx - 1) * g.dx, (ny - 1) * g.dy, (nz - 1) * g.dz, g.dx, g.dy,
+                            g.dz)
+    pb.state = init_particles(n_particles, pb.grid, 3.0, seed=5)
+    return pb
+
+
+@pytest.mark.parametrize("shape", [(20, 20, 20), (20, 12, 33), (33, 9, 17), (100, 8, 8)])
+@pytest.mark.parametrize("sort_every,periodic", [(0, True), (16, True), (16, False)])
+def test_fp64_bricks_with_offset_tables_bit_exact(cuda, shape, sort_every, periodic):
+    """The FP64 push over bricks whose node offsets come from tables: unsorted and sorted, periodic and open, against
+    the oracle."""
+    pb = _table_problem(shape, 700)
+    (mu_o, ac_o, st_o, al_o), (col, ac_g, st_g, al_g) = run_both(pb, 129, 4, "mu", periodic=periodic,
+                                                                 storage="brick_f64", sort_every=sort_every)
+    assert np.array_equal(col.mu, mu_o, equal_nan=True)
+    assert np.array_equal(ac_g, ac_o) and np.array_equal(al_g, al_o)
+    for k in R.KEYS:
+        assert np.array_equal(st_g[k], st_o[k], equal_nan=True), k
+
+
+@pytest.mark.parametrize("n", [5, 148 * 32 + 1, 148 * 512 + 1])
+def test_fp64_bricks_with_offset_tables_particle_counts(cuda, n):
+    """The same at the edges of the launch shape."""
+    (mu_o, _, st_o, _), (col, _, st_g, _) = run_both(_table_problem((20, 12, 33), n), 13, 3, "mu", storage="brick_f64")
+    assert np.array_equal(mu_o, col.mu, equal_nan=True)
+    for k in R.KEYS:
+        assert np.array_equal(st_o[k], st_g[k]), k
