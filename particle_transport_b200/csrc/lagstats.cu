@@ -42,6 +42,7 @@ constexpr int kDppThreads = 512;
 constexpr int kDppWarps = kDppThreads / kWarp;
 constexpr int kDppLags = 4;    // lags of a set: |p|[s] is read once for them
 constexpr int kDppUnroll = 2;  // starts per lane and pass
+constexpr int kDppStage = 4;   // pairs of saves that a thread stages side by side
 
 struct DppLaunch {
     const double* pmag;    // [n][pitch] |p| of this launch's particles
@@ -49,7 +50,8 @@ struct DppLaunch {
     const int64_t* lags;
     int nl;
     int ppc;       // particle series per CTA
-    int sets;      // lag sets, a multiple of the warps
+    int sets;      // lag sets: a divisor or a multiple of the warps
+    int qparts;    // warps of a set that share a tile's particles; the others share the starts
     int first;     // 1: set the partials, 0: add to them
     DppPart* part; // [grid][nl]
 };
@@ -90,27 +92,28 @@ __global__ void __launch_bounds__(256) pmag_kernel(const float* __restrict__ mom
 }
 
 struct DppFixed {
-    size_t sd2, cnt, sorted, idx, nfin, fin, series;
+    size_t sd2, cnt, sorted, idx, nfin, bad, series;
 };
 __host__ __device__ inline DppFixed dpp_fixed(int sets, int nl, int ppc)
 {
     auto a16 = [](size_t v) { return (v + 15) & ~(size_t)15; };
     DppFixed f;
-    f.sd2 = (size_t)sets * kDppLags * sizeof(double);
+    f.sd2 = (size_t)(sets > kDppWarps ? sets : kDppWarps) * kDppLags * sizeof(double);
     f.cnt = 2 * f.sd2;
     f.sorted = f.cnt + sizeof(unsigned long long) * nl;
     f.idx = f.sorted + sizeof(int) * nl;
     f.nfin = f.idx + sizeof(int) * nl;
-    f.fin = f.nfin + sizeof(int) * ppc;
-    f.series = a16(f.fin + sizeof(int) * ppc);
+    f.bad = f.nfin + sizeof(int) * ppc;
+    f.series = a16(f.bad + sizeof(int) * ppc);
     return f;
 }
 
-// Starts [s0, s1) against NL lags: p[s + L[k]] - p[s], added to sd[k] and sq[k].
+// Starts [s0, s1) against NL lags: p[s + L[k]] - p[s], added to sd[k] and sq[k]; the
+// lanes of a pass take the starts from `lane` on, the next pass is `hop` on.
 // TEST: only finite differences count (into cnt).  Starts are unsigned: a series may
 // hold nearly 2^31 saves, and the loops look a pass past the end.
 template <int NL, bool TEST>
-__device__ __forceinline__ void dpp_rows(const double* __restrict__ p, unsigned s0, unsigned s1, const int (&L)[kDppLags], int lane,
+__device__ __forceinline__ void dpp_rows(const double* __restrict__ p, unsigned s0, unsigned s1, const int (&L)[kDppLags], int lane, int hop,
                                          double (&sd)[kDppLags], double (&sq)[kDppLags], int (&cnt)[kDppLags])
 {
     auto pair = [&](double ps, double pe, int k) {
@@ -124,7 +127,7 @@ __device__ __forceinline__ void dpp_rows(const double* __restrict__ p, unsigned 
         sq[k] = fma(d, d, sq[k]);
     };
     unsigned s = s0 + lane;
-    for (; s + (kDppUnroll - 1) * kWarp < s1; s += kDppUnroll * kWarp) {
+    for (; s + (kDppUnroll - 1) * kWarp < s1; s += hop) {
         double ps[kDppUnroll], pe[kDppUnroll][NL];
 #pragma unroll
         for (int u = 0; u < kDppUnroll; ++u) {
@@ -137,19 +140,21 @@ __device__ __forceinline__ void dpp_rows(const double* __restrict__ p, unsigned 
 #pragma unroll
             for (int k = 0; k < NL; ++k) pair(ps[u], pe[u][k], k);
     }
-    for (; s < s1; s += kWarp) {
+    if (s < s1) {  // at most the last pass of a lane is not whole
         const double ps = p[s];
 #pragma unroll
         for (int k = 0; k < NL; ++k) pair(ps, p[s + L[k]], k);
     }
 }
+static_assert(kDppUnroll == 2, "dpp_rows ends with one start per lane");
 
 // Lags are dealt to sets of at most kDppLags, in the order of their value back and
 // forth over the sets, so that the sets have about equal numbers of pairs; a warp
-// owns a set (or every 16th) for all particles, its lanes take consecutive starts,
-// and the lanes' sums are added across the warp once per tile of particles.  A
-// warp's 8-byte |p| reads are consecutive (no bank conflicts, whatever the lags),
-// and |p|[s] is read once for the set's lags.
+// owns a set (or every 16th), its lanes take consecutive starts, and the lanes' sums
+// are added across the warp once per tile of particles.  A warp's 8-byte |p| reads
+// are consecutive (no bank conflicts, whatever the lags), and |p|[s] is read once for
+// the set's lags.  Up to 32 lags fill fewer sets than there are warps: the sets stay
+// full, and 2 to 16 warps share one, by particles or by starts.
 //
 // A particle whose finite saves are a prefix [0, nfin) needs no test in the pair
 // loop: the starts below nfin - L are exactly lag L's pairs, so a set runs its
@@ -157,30 +162,34 @@ __device__ __forceinline__ void dpp_rows(const double* __restrict__ p, unsigned 
 // so on, and the count of a lag is max(0, nfin - L).  Other particles take the same
 // loops up to nsave - L with a finite test per pair.
 //
-// A set's sums have one writer and CTAs are added in order: the result is
-// deterministic.
+// A warp's sums have one writer, and the warps of a set and the CTAs are added in
+// order: the result is deterministic.
 //
 // Bound by shared-memory bandwidth: 8 bytes per pair and 8 per start and set,
 // about 2.6 cycles of the SM's 128 B/clk per 32 pairs, with the FP64 pipe at 1.5.
 // Two CTAs per SM, so that one's staging runs under the other's pairs.
 // 65,536 x 4001 saves x 55 lags with 16 energy snapshots and histograms: 8.45 ms
 // with two lags per pass, a finite test per pair and the reads of the momenta in
-// this kernel; 5.75 ms now (4.85 ms here, 0.85 ms in pmag_kernel).
+// this kernel; 5.60 ms now (0.85 ms of it in pmag_kernel).  With few lags or short
+// series the staging counts: a series at a time, with the finite saves counted, it
+// is a chain of load latencies.  65,536 x 201 saves, 1 and 18 lags: 0.45 and 0.50 ms
+// that way with one lag per warp, 0.18 and 0.28 now (0.06 in pmag_kernel); x 801
+// saves, 4 lags: 0.74 and 0.45.
 template <bool SMEM_SLOTS>
 __global__ void __launch_bounds__(kDppThreads, 2) dpp_kernel(DppLaunch a)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const int nl = a.nl, nsave = (int)a.nsave, ppc = a.ppc, sets = a.sets;
     const DppFixed F = dpp_fixed(sets, nl, ppc);
-    double* acc_sd = (double*)smem;  // [set][kDppLags]
+    double* acc_sd = (double*)smem;  // [part][set][kDppLags]
     double* acc_sd2 = (double*)(smem + F.sd2);
     unsigned long long* acc_cnt = (unsigned long long*)(smem + F.cnt);  // [lag, by value]
     int* s_lag = (int*)(smem + F.sorted);  // ascending; nsave where no pair exists
     int* s_idx = (int*)(smem + F.idx);     // index of the lag in a.lags
     int* s_nfin = (int*)(smem + F.nfin);   // first non-finite save
-    int* s_fin = (int*)(smem + F.fin);     // finite saves
+    int* s_bad = (int*)(smem + F.bad);     // saves that are not finite
     double* series = (double*)(smem + F.series);  // [ppc][pitch]
-    for (int i = threadIdx.x; i < sets * kDppLags; i += blockDim.x) acc_sd[i] = acc_sd2[i] = 0.0;
+    for (int i = threadIdx.x; i < max(sets, kDppWarps) * kDppLags; i += blockDim.x) acc_sd[i] = acc_sd2[i] = 0.0;
     for (int i = threadIdx.x; i < nl; i += blockDim.x) {
         acc_cnt[i] = 0ull;
         auto value = [&](int q) {  // the range test in 64 bits, before the narrowing
@@ -200,6 +209,10 @@ __global__ void __launch_bounds__(kDppThreads, 2) dpp_kernel(DppLaunch a)
     const int warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
     // lag k of a set, by value: rows of `sets` lags dealt forth and back
     auto dealt = [&](int set, int k) { return k * sets + (k & 1 ? sets - 1 - set : set); };
+    // fewer sets than warps: `parts` warps share a set
+    const int across = min(sets, kDppWarps), parts = kDppWarps / across, part = warp / across;
+    const int from_start = part / a.qparts * (kDppUnroll * kWarp) + lane;
+    const int hop = parts / a.qparts * (kDppUnroll * kWarp);
     const int64_t tiles = (a.n + ppc - 1) / ppc;
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const int64_t p0 = tile * ppc;
@@ -207,38 +220,47 @@ __global__ void __launch_bounds__(kDppThreads, 2) dpp_kernel(DppLaunch a)
         const double* from = a.pmag + p0 * a.pitch;
         for (int i = threadIdx.x; i < ppc; i += blockDim.x) {
             s_nfin[i] = nsave;
-            s_fin[i] = 0;
+            s_bad[i] = 0;
         }
         __syncthreads();
-        for (int q = 0; q < np; ++q) {
-            int bad = nsave, fin = 0;
-            auto look = [&](double v, int s) {
-                if (s >= nsave) return;
-                if (isfinite(v)) ++fin;
-                else bad = min(bad, s);
-            };
-            // two saves at a time: the pitch is even and the rows 16-byte aligned
-            const double2* row = (const double2*)(from + q * a.pitch);
-#pragma unroll 4
-            for (int i = threadIdx.x; i < (int)(a.pitch / 2); i += blockDim.x) {
-                const double2 v = row[i];
-                if (SMEM_SLOTS) ((double2*)(series + q * a.pitch))[i] = v;
-                look(v.x, 2 * i);
-                look(v.y, 2 * i + 1);
-            }
-            if (bad < nsave) atomicMin(&s_nfin[q], bad);
+        // the tile is one run of memory, copied two saves at a time (the pitch is even
+        // and the rows 16-byte aligned) whatever the length of a series; which
+        // particle a save belongs to matters only where it is not finite
+        const int half = (int)(a.pitch / 2), all = np * half;
+        const double2* row = (const double2*)from;
+        for (int i0 = warp * kWarp + lane; i0 - lane < all; i0 += kDppStage * kDppThreads) {
+            double2 v[kDppStage];
 #pragma unroll
-            for (int o = kWarp / 2; o > 0; o >>= 1) fin += __shfl_xor_sync(0xffffffffu, fin, o);
-            if (lane == 0) atomicAdd(&s_fin[q], fin);
+            for (int k = 0; k < kDppStage; ++k) {
+                const int i = i0 + k * kDppThreads;
+                v[k] = i < all ? row[i] : make_double2(0.0, 0.0);
+            }
+#pragma unroll
+            for (int k = 0; k < kDppStage; ++k) {
+                const int i = i0 + k * kDppThreads;
+                if (SMEM_SLOTS && i < all) ((double2*)series)[i] = v[k];
+                const bool bx = !isfinite(v[k].x), by = !isfinite(v[k].y);
+                if (!__any_sync(0xffffffffu, bx || by)) continue;
+                const int q = min(i, all - 1) / half, s = 2 * (i - q * half);
+                const bool y = by && s + 1 < nsave;  // the pad of an odd series is no save
+                // the lanes of a particle add their counts up first
+                const unsigned same = __match_any_sync(0xffffffffu, q);
+                const int n = __reduce_add_sync(same, (int)bx + (int)y);
+                const int first = __reduce_min_sync(same, bx ? s : (y ? s + 1 : nsave));
+                if (n > 0 && lane == __ffs(same) - 1) {
+                    atomicAdd(&s_bad[q], n);
+                    atomicMin(&s_nfin[q], first);
+                }
+            }
         }
         __syncthreads();
         for (int l = threadIdx.x; l < nl; l += blockDim.x) {
             long long c = 0;
             for (int q = 0; q < np; ++q)
-                if (s_fin[q] == s_nfin[q]) c += max(0, s_nfin[q] - s_lag[l]);
+                if (nsave - s_bad[q] == s_nfin[q]) c += max(0, s_nfin[q] - s_lag[l]);
             if (c > 0) atomicAdd(&acc_cnt[l], (unsigned long long)c);
         }
-        for (int set = warp; set < sets; set += kDppWarps) {
+        for (int set = warp % across; set < sets; set += kDppWarps) {
             int L[kDppLags], cnt[kDppLags];
             double sd[kDppLags], sq[kDppLags];
 #pragma unroll
@@ -248,23 +270,23 @@ __global__ void __launch_bounds__(kDppThreads, 2) dpp_kernel(DppLaunch a)
                 cnt[k] = 0;
                 sd[k] = sq[k] = 0.0;
             }
-            for (int q = 0; q < np; ++q) {
-                const bool prefix = s_fin[q] == s_nfin[q];
+            for (int q = part % a.qparts; q < np; q += a.qparts) {
+                const bool prefix = nsave - s_bad[q] == s_nfin[q];
                 const int end = prefix ? s_nfin[q] : nsave;
                 int lim[kDppLags];  // falls with k
 #pragma unroll
                 for (int k = 0; k < kDppLags; ++k) lim[k] = max(0, end - L[k]);
                 const double* p = (SMEM_SLOTS ? (const double*)series : from) + q * a.pitch;
                 if (prefix) {
-                    dpp_rows<4, false>(p, 0, lim[3], L, lane, sd, sq, cnt);
-                    dpp_rows<3, false>(p, lim[3], lim[2], L, lane, sd, sq, cnt);
-                    dpp_rows<2, false>(p, lim[2], lim[1], L, lane, sd, sq, cnt);
-                    dpp_rows<1, false>(p, lim[1], lim[0], L, lane, sd, sq, cnt);
+                    dpp_rows<4, false>(p, 0, lim[3], L, from_start, hop, sd, sq, cnt);
+                    dpp_rows<3, false>(p, lim[3], lim[2], L, from_start, hop, sd, sq, cnt);
+                    dpp_rows<2, false>(p, lim[2], lim[1], L, from_start, hop, sd, sq, cnt);
+                    dpp_rows<1, false>(p, lim[1], lim[0], L, from_start, hop, sd, sq, cnt);
                 } else {
-                    dpp_rows<4, true>(p, 0, lim[3], L, lane, sd, sq, cnt);
-                    dpp_rows<3, true>(p, lim[3], lim[2], L, lane, sd, sq, cnt);
-                    dpp_rows<2, true>(p, lim[2], lim[1], L, lane, sd, sq, cnt);
-                    dpp_rows<1, true>(p, lim[1], lim[0], L, lane, sd, sq, cnt);
+                    dpp_rows<4, true>(p, 0, lim[3], L, from_start, hop, sd, sq, cnt);
+                    dpp_rows<3, true>(p, lim[3], lim[2], L, from_start, hop, sd, sq, cnt);
+                    dpp_rows<2, true>(p, lim[2], lim[1], L, from_start, hop, sd, sq, cnt);
+                    dpp_rows<1, true>(p, lim[1], lim[0], L, from_start, hop, sd, sq, cnt);
                 }
             }
 #pragma unroll
@@ -276,8 +298,8 @@ __global__ void __launch_bounds__(kDppThreads, 2) dpp_kernel(DppLaunch a)
                     cnt[k] += __shfl_xor_sync(0xffffffffu, cnt[k], o);
                 }
                 if (lane == 0) {
-                    acc_sd[set * kDppLags + k] += sd[k];
-                    acc_sd2[set * kDppLags + k] += sq[k];
+                    acc_sd[(part * sets + set) * kDppLags + k] += sd[k];
+                    acc_sd2[(part * sets + set) * kDppLags + k] += sq[k];
                     const int l = dealt(set, k);
                     if (l < nl && cnt[k] > 0) atomicAdd(&acc_cnt[l], (unsigned long long)cnt[k]);
                 }
@@ -289,7 +311,11 @@ __global__ void __launch_bounds__(kDppThreads, 2) dpp_kernel(DppLaunch a)
         const int l = dealt(i / kDppLags, i % kDppLags);
         if (l >= nl) continue;
         DppPart& out = a.part[(int64_t)blockIdx.x * nl + s_idx[l]];
-        DppPart r{(long long)acc_cnt[l], acc_sd[i], acc_sd2[i]};
+        DppPart r{(long long)acc_cnt[l], 0.0, 0.0};
+        for (int q = 0; q < parts; ++q) {
+            r.sdp += acc_sd[q * sets * kDppLags + i];
+            r.sdp2 += acc_sd2[q * sets * kDppLags + i];
+        }
         if (!a.first) {
             r.count += out.count;
             r.sdp += out.sdp;
@@ -617,7 +643,9 @@ int run_dpp(pt_ctx* ctx, const DppArgs& a, cudaStream_t s)
     for (int lag0 = 0; lag0 < a.n_lags; lag0 += nl_cap) {
         const int nl = std::min(nl_cap, a.n_lags - lag0);
         DppLaunch L;
-        L.sets = kDppWarps * ((nl + kDppWarps * kDppLags - 1) / (kDppWarps * kDppLags));
+        L.sets = 1;
+        while (L.sets < kDppWarps && L.sets * kDppLags < nl) L.sets *= 2;
+        if (L.sets == kDppWarps) L.sets *= (nl + kDppWarps * kDppLags - 1) / (kDppWarps * kDppLags);
         // Series on chip when they fit, two CTAs per SM when half of it holds one
         // (the reserved KB per CTA left out).  As many as fit, up to 16, but no
         // more than gives every CTA of the chip a tile.
@@ -629,6 +657,19 @@ int run_dpp(pt_ctx* ctx, const DppArgs& a, cudaStream_t s)
         while (smem_slots && ppc < 16 && (int64_t)ppc * ctx->num_sms * (two ? 2 : 1) < a.chunk &&
                need(ppc + 1) <= (two ? half : (size_t)max_smem))
             ++ppc;
+        // the warps of a set share particles or starts, whichever leaves the busiest the
+        // fewest passes
+        const int parts = std::max(1, kDppWarps / L.sets);
+        int64_t least = 0;
+        L.qparts = 1;
+        for (int q = 1; q <= parts; q *= 2) {
+            const int64_t hop = (int64_t)kDppUnroll * kWarp * (parts / q);
+            const int64_t passes = ((ppc + q - 1) / q) * ((a.nsave + hop - 1) / hop);
+            if (q == 1 || passes <= least) {
+                least = passes;
+                L.qparts = q;
+            }
+        }
         const size_t smem = smem_slots ? need(ppc) : dpp_fixed(L.sets, nl, ppc).series;
         void* kfn = smem_slots ? (void*)dpp_kernel<true> : (void*)dpp_kernel<false>;
         PT_CUDA(allow_smem(kfn, smem));

@@ -541,3 +541,14 @@ def test_dpp_on_a_full_device(cuda):
         assert close(got["sum_delta_p_norm"], want["sum_delta_p_norm"], scale=scale)
     del graph
     ctx.close()
+
+
+# 1, 2, 4 and 8 lag sets, whose 16, 8, 4 and 2 warps share the particles of a tile or the starts of a series; series
+# shorter than a warp (several in one warp's copies), tiles with a remainder, an even and an odd number of saves
+@pytest.mark.parametrize("chunk,nsave,n_lags,pattern", [
+    (4801, 9, 1, "mixed"), (5000, 40, 2, "mixed"), (4999, 201, 5, "holes"), (700, 3000, 2, "dead"),
+    (2999, 900, 14, "mixed"), (301, 4001, 27, "holes"), (2, 30001, 3, "mixed"), (4737, 64, 30, "none"),
+])
+def test_dpp_few_lags(cuda, oracle, chunk, nsave, n_lags, pattern):
+    """As test_dpp_shapes_and_nan_patterns, where a set of lags has several warps."""
+    test_dpp_shapes_and_nan_patterns(cuda, oracle, chunk, nsave, n_lags, pattern)
