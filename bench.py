@@ -84,6 +84,7 @@ def parse():
     ap.add_argument("--precision-grid", type=int, default=256)
     ap.add_argument("--precision-particles", type=int, default=1_048_576)
     ap.add_argument("--precision-gyroperiods", type=int, default=200)
+    ap.add_argument("--details", default="", help="file for the whole result, the printed line's legs in full")
     return ap.parse_args()
 
 
@@ -704,12 +705,38 @@ def run_ours(args, ws, rank, local):
                 "job_latency": ({"p50_s": serving["p50_s"], "p99_s": serving["p99_s"], "jobs": serving["jobs"]}
                                 if serving and "p50_s" in serving else None),
                 "serving": serving, "config1_end_to_end": config1, "precision": precision}
-        print(json.dumps(line), flush=True)
+        if args.details:
+            with open(args.details, "w") as f:
+                json.dump(line, f, indent=1)
+        print(json.dumps(compact(line)), flush=True)
+
+
+# legs of the result that the printed line gives by a few numbers each, and what those are; the rest (sizes, texts,
+# per-case values) is in the file of --details
+LEGS = ("fp32_bricks", "fp64_push", "lag_pairs", "dpp", "batched", "serving", "config1_end_to_end", "precision")
+FIGURES = ("value", "ms_per_pass", "frac", "cores", "lag_pairs_per_s", "p50_s", "p99_s", "busy_rate", "rate",
+           "gpu_f64_s", "gpu_f32_bf16_s", "cpu_oracle_s", "within_tolerance", "D_mumu", "delta_mu2", "D_pp",
+           "bricks", "roofline", "cpu_baseline", "phase_space_dmumu", "matched_batch", "max_rel_err_resolved", "f32",
+           "bf16", "error")
+
+
+def compact(line: dict) -> dict:
+    """The result as printed, a line of at most 3,000 characters: everything outside the legs, and of a leg its
+    figures to five digits."""
+    def figures(v):
+        if isinstance(v, dict):
+            inner = {k: figures(w) for k, w in v.items() if k in FIGURES}
+            return {k: w for k, w in inner.items() if w != {}}
+        if isinstance(v, str):  # an error
+            return v[:100]
+        return float(f"{v:.5g}") if isinstance(v, float) else v
+
+    return {k: figures(v) if k in LEGS else v for k, v in line.items()}
 
 
 # Warp instructions per lag pair of the statistics kernels: smsp__inst_executed.sum
 # of one launch over the pairs it processed, from an ncu capture of the bench's
-# small case (profiles/dmumu_*.md, profiles/dpp_*.md).  These kernels are
+# small case (kept under profiles/).  These kernels are
 # bound by instruction issue, whose ceiling is one warp instruction per cycle
 # per SM sub-partition (4 per SM).
 # D_pp counts its two kernels (pmag_kernel and dpp_kernel).

@@ -37,3 +37,29 @@ def test_reference_arm_line():
 def test_reference_arm_other_ranks_exit_without_work():
     r = _run({"WORLD_SIZE": "2", "RANK": "1", "LOCAL_RANK": "1"})
     assert r.returncode == 0 and not [l for l in r.stdout.splitlines() if l.startswith("{")]
+
+
+def test_printed_line_is_compact():
+    """The printed line keeps the contract's keys as they are and stays short however long the legs get."""
+    sys.path.insert(0, ROOT)
+    import bench
+
+    contract = {"metric": bench.METRIC, "value": 5.5491234567e10, "unit": bench.UNIT, "ms_per_step": 19.3512345678,
+                "config": {"workload": "w" * 150}, "roofline": {"kernel": "k", "frac": 0.123456789},
+                "e2e": {"value": 1.23456789e10, "unit": "u", "h2d_bytes_per_step": 7}, "clocks": {"reasons": []},
+                "job_latency": {"p50_s": 0.123456789}, "gpu_launches": 100}
+    per_case = {f"mode{i}/{e}GeV": {f"form{f}": {f"product{q}": 0.123456789 for q in range(3)} for f in range(9)}
+                for i in range(4) for e in (1, 10, 100)}
+    leg = {"value": 1.23456789e11, "unit": "u" * 40, "note": "n" * 400, "roofline": {"frac": 0.87654321, "note": "x" * 80},
+           "per_campaign": [{"n": 1}] * 50}
+    line = dict(contract, **{k: leg for k in bench.LEGS[:-1]},
+                precision={"max_rel_err_resolved": {"f32": {"D_mumu": 0.001234567}}, "within_tolerance": True,
+                           "per_case": per_case, "criterion": "c" * 500})
+    assert len(json.dumps(line)) > 12000
+    out = bench.compact(line)
+    assert len(json.dumps(out)) < 3000
+    for k, v in contract.items():
+        assert out[k] == v, k
+    assert out["lag_pairs"] == {"value": 1.2346e11, "roofline": {"frac": 0.87654}}
+    assert out["precision"] == {"max_rel_err_resolved": {"f32": {"D_mumu": 0.0012346}}, "within_tolerance": True}
+    assert bench.compact(dict(contract, serving=None))["serving"] is None
