@@ -60,6 +60,7 @@ CallMem::CallMem(pt_ctx* ctx, size_t bytes, cudaStream_t s) : s_(s)
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     cudaError_t e = cudaStreamIsCapturing(s, &cap);
     if (e == cudaSuccess && cap != cudaStreamCaptureStatusNone) return;
+    RelaxedCapture relaxed;
     if (e == cudaSuccess && !ctx->pool) {
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;

@@ -146,12 +146,26 @@ int scratch_get(pt_ctx* ctx, int slot, size_t bytes, void** out);
 // path that needs none.  The context's pool holds at most kPoolKeep bytes of it
 // between calls.
 constexpr uint64_t kPoolKeep = 256u << 20;
+// The thread's calls, while one lives, do not end a capture that runs on some other
+// stream: by default an allocation ends every capture begun in the global mode.
+class RelaxedCapture {
+public:
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+    RelaxedCapture(const RelaxedCapture&) = delete;
+    RelaxedCapture& operator=(const RelaxedCapture&) = delete;
+
+private:
+    cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+};
 class CallMem {
 public:
     CallMem(pt_ctx* ctx, size_t bytes, cudaStream_t s);
     ~CallMem()
     {
-        if (p_) cudaFreeAsync(p_, s_);
+        if (!p_) return;
+        RelaxedCapture relaxed;
+        cudaFreeAsync(p_, s_);
     }
     CallMem(const CallMem&) = delete;
     CallMem& operator=(const CallMem&) = delete;
@@ -287,7 +301,8 @@ inline bool fast_storage(int storage)
 
 // Node offsets of power-of-two cubes, whose nodes and bricks are both in Morton
 // order (pt_field.morton): offx = morton10, offy = 2 morton10, offz = 4 morton10.
-// every third bit, and the bits of v < 1024 spread to them
+// every third bit, and the bits of v < 1024 spread to them (the multiply-and-mask
+// spread of Karras, "Thinking Parallel, Part III", 2012)
 constexpr uint32_t kMorton = 0x09249249u;
 __device__ __forceinline__ uint32_t morton10(uint32_t v)
 {

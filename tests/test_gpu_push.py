@@ -506,3 +506,38 @@ def test_fp64_bricks_with_offset_tables_particle_counts(cuda, n):
     assert np.array_equal(mu_o, col.mu, equal_nan=True)
     for k in R.KEYS:
         assert np.array_equal(st_o[k], st_g[k]), k
+
+
+def test_export_beside_a_capture(cuda):
+    """An export of a large sorted state on a stream of its own, the first of its context and one more, leaves a
+    capture that runs on another stream alone."""
+    torch = cuda
+    from particle_transport_b200 import _lib
+    n = (1 << 21) + 5
+    pb = small_problem(n=16, n_particles=1000, u_over_c=1e-4, energy_GeV=3.0)
+    st = {k: torch.as_tensor(np.resize(v, n), device="cuda") for k, v in pb.state.items()}
+    alive = torch.ones(n, dtype=torch.uint8, device="cuda")
+    alive[::3] = 0
+    ens = R.FastEnsemble(FieldLibrary(pb.fields, pb.grid, "brick_bf16"), st, alive)
+    ens.sort()
+    want, _ = ens.export()
+    out = {k: torch.empty(n, dtype=torch.float64, device="cuda") for k in R.KEYS}
+    al = torch.empty(n, dtype=torch.uint8, device="cuda")
+    ctx = _lib.Context(0)
+    x = torch.arange(10, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = x + 1
+        for _ in range(2):
+            _lib.call("pt_fast_state_export", ctx.handle, ens.handle, *[_lib.ptr(out[k]) for k in R.KEYS],
+                      _lib.ptr(al))
+        z = y * 2
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(z, 2 * (x + 1)) and torch.equal(al, alive)
+    for k in R.KEYS:
+        assert torch.equal(out[k], want[k]), k
+    del graph
+    ctx.close()
+    ens.close()
