@@ -22,8 +22,8 @@
 // hist2 over k are the counts.  Other particles take a loop that tests the
 // partner and counts pairs.
 //
-// What bounds it: instruction issue (60 % busy at 16 warps per SM) with the
-// shared-memory pipe (67 %) and the conversion pipe (48 %) close behind; a pair
+// What bounds it: instruction issue (63 % busy at 16 warps per SM) with the
+// shared-memory pipe (69 %) and the conversion pipe (50 %) close behind; a pair
 // row costs an address add, a load, a conversion, two adds and an FMA.  131,072
 // x 4001 saves x 55 lags x 50 bins: 28.2 ms with one lag per lane, 15.1 ms now
 // (1.6e12 pairs/s); 4096 x 801 x 19 x 20: 263 us, 147 us now.
@@ -1124,6 +1124,9 @@ int run_dmumu_t(const PartSource& src, const DmumuArgs& a, const MuT* mu, int64_
         }
         PT_CUDA(allow_smem(kfn, smem));
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, threads, smem);
+        // one CTA per SM where the series are in global memory, as the bound of the
+        // scratch that callers are given counts on (registers allow no second one anyway)
+        if (!a.injection && h.mode == SLOT_GLOBAL) per_sm = 1;
         blocks = std::min<int64_t>(blocks, (int64_t)ctx->num_sms * std::max(1, per_sm));
         if (src.fixed) {
             const size_t per_cta = (size_t)nl * a.n_bins * 24 + sizeof(WelfordPart) * (size_t)nl + 64;

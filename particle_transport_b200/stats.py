@@ -297,8 +297,10 @@ def dmumu_noalloc_fits(nsave: int, n_lags: int, n_bins: int) -> bool:
 
 def dmumu_scratch_bound(nsave: int, n_lags: int, n_bins: int, num_sms: int = 148) -> int:
     """Upper bound of the device scratch pt_dmumu_accumulate_device asks its
-    context for when the series are staged in global memory (1024-thread
-    CTAs, at most two per SM, eight series per CTA)."""
+    context for when the series are staged in global memory: one CTA per SM
+    with at most eight series, 8 bytes per save (a Float32 value and a 4-byte
+    list entry).  It counts two CTAs per SM with the slots of the on-chip
+    form, 6 bytes per save at least."""
     if n_lags <= 0:
         return 0
     nl, slot, _ = _dmumu_shape(nsave, n_lags, n_bins)
