@@ -740,7 +740,7 @@ def compact(line: dict) -> dict:
 # bound by instruction issue, whose ceiling is one warp instruction per cycle
 # per SM sub-partition (4 per SM).
 # D_pp counts its two kernels (pmag_kernel and dpp_kernel).
-WARP_INST_PER_PAIR = {"dmumu_kernel": 21.777e9 / 49.193e9, "dpp_kernel": (2.861e9 + 0.771e9) / 12.298e9}
+WARP_INST_PER_PAIR = {"dmumu_kernel": 21.777e9 / 49.193e9, "dpp_kernel": (146.511e6 + 41.796e6) / (3552 * 187657)}
 
 
 def issue_roofline(kernel: str, pairs_per_s: float, clocks, device) -> dict:

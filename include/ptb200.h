@@ -6,7 +6,7 @@
  * Each entry point below names the reference function (file:line, paths in
  * the reference project) whose body it replaces; the Julia host keeps the
  * function's signature, its HDF5 I/O and its config handling and calls the
- * library through ccall (see INTEGRATION.md for the bindings).
+ * library through ccall (julia/PtB200.jl has the bindings).
  *
  * Conventions
  *  - Every function returns PT_OK (0) or a negative PT_ERR_* code; the

@@ -469,7 +469,7 @@ struct BSource {
 // instruction.  The kernel is bound by the L1's queue of requests that miss, one per
 // line and instruction: with each lane reading its own record in 32-byte loads that
 // queue was full (a third of all stalls) at 41 % of the DRAM bandwidth; now DRAM is
-// 72 % busy.  256^3, 65,536 particles x 801 saves, FP32: 3.20 ms, 2.00 ms now.
+// 75 % busy.  256^3, 65,536 particles x 801 saves, FP32: 3.20 ms, 2.00 ms now.
 template <typename R>
 constexpr int kPsRows = sizeof(R) == 4 ? 8 : 4;  // 32-byte runs of a particle's mu
 

@@ -663,12 +663,13 @@ int pt_push_run(pt_ctx* ctx, const pt_field* f, double* x1, double* x2, double* 
     // transpose turns each chunk into the rows the callback receives.
     const bool tf = p->precision == PT_PUSH_F32 && p->cache_mode == PT_CACHE_MU && !p->cache_f64 && n > 0;
     const int tf_pitch = 8;
-    // Rows per egress chunk: the rows of 64 steps (one launch), so that the rows of
-    // one chunk are handed over while the next chunks run -- a 256-step run in one
-    // chunk pushed first and handed over all its rows after that (65,536
-    // particles, FP64, phase space: 8.7 ms, 6.4 in four chunks) -- with bounded
-    // staging memory.  The sorted FP64 push copies and sorts the state once per
-    // chunk: 256 steps.
+    // Rows per egress chunk: the rows of 64 steps, up to the next save, so that the
+    // rows of one chunk are handed over while the next chunks run -- a 256-step run in
+    // one chunk pushed first and handed over all its rows after that (65,536
+    // particles, FP64, phase space: 9.7 ms, 7.65 in four chunks) -- with bounded
+    // staging memory.  (Strides that do not divide 64 add a launch of a few steps per
+    // chunk; rounding down to whole launches measured the same at strides 3, 5 and 10.)
+    // The sorted FP64 push copies and sorts the state once per chunk: 256 steps.
     const bool resort = p->precision == PT_PUSH_F64 && f->storage == PT_FIELD_BRICK_F64 && p->sort_every > 0;
     const int64_t steps_per_chunk = resort ? 256 : 64;
     int64_t R = tf ? tf_pitch : std::max<int64_t>(1, (steps_per_chunk + stride - 1) / stride);
