@@ -25,6 +25,7 @@ struct pt_batch {
     BatchCampaignDev* d_camps = nullptr;
     std::vector<BatchCampaignDev> h_camps;
     std::vector<const pt_field*> fields;
+    std::vector<int64_t> field_bytes;  // of each campaign's field, when it was added
     BatchTile* d_tiles = nullptr;
     int* d_ntiles = nullptr;
     int* d_counter = nullptr;
@@ -114,7 +115,7 @@ void deal_tiles(pt_batch* b)
     std::vector<BatchTile>& tiles = b->tile_scratch;
     std::vector<int32_t>& first = b->bucket_scratch;
     struct Group {  // the running campaigns of a field
-        const pt_field* field;
+        const void* nodes;
         bool dealt;
         int64_t buckets, base;  // tiles of the largest campaign if dealt, of all otherwise; first bucket
     };
@@ -128,10 +129,10 @@ void deal_tiles(pt_batch* b)
     for (int c = 0; c < b->max_camps; ++c) {
         const BatchCampaignDev& C = b->h_camps[c];
         if (!C.active || !C.running) continue;
-        const pt_field* field = b->fields[c];
         size_t f = 0;
-        while (f < groups.size() && groups[f].field != field) ++f;
-        if (f == groups.size()) groups.push_back(Group{field, field->bytes > 2 * b->l2_bytes, 0, 0});
+        while (f < groups.size() && groups[f].nodes != C.a.fld.nodes) ++f;
+        if (f == groups.size())
+            groups.push_back(Group{C.a.fld.nodes, b->field_bytes[(size_t)c] > 2 * b->l2_bytes, 0, 0});
         Group& G = groups[f];
         const int64_t T = campaign_tiles(C);
         place[(size_t)c] = Place{(int)f, G.dealt ? 0 : G.buckets};
@@ -311,6 +312,7 @@ int pt_batch_create(pt_ctx* ctx, int64_t capacity, int max_campaigns, int storag
     b->sort = sort ? 1 : 0;
     b->h_camps.assign(max_campaigns, BatchCampaignDev{});
     b->fields.assign(max_campaigns, nullptr);
+    b->field_bytes.assign(max_campaigns, 0);
     int l2 = 0;
     cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, ctx->device);
     b->l2_bytes = l2;
@@ -447,6 +449,7 @@ int pt_batch_add(pt_ctx* ctx, pt_batch* b, const pt_campaign_desc* d, int* id)
     C.running = 1;
     b->h_camps[c] = C;
     b->fields[c] = f;
+    b->field_bytes[c] = f->bytes;
     const int words = (int)(g.nx + g.ny + g.nz);
     if (words > b->smem_words) {
         b->smem_words = words;
