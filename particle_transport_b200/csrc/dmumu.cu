@@ -262,12 +262,15 @@ __device__ __forceinline__ T start_sum(const T (&v)[NS], int q0, int j)
     return (odd ? b : a) + __shfl_xor_sync(0xffffffffu, odd ? a : b, kLagLanes);
 }
 
+// Saves and list positions in loops that run up to some blocks past the end: unsigned
+// where a series may hold nearly 2^31 saves, in global memory; at most 65,535 are on
+// chip.
+template <int MODE>
+using SavePos = std::conditional_t<MODE == SLOT_GLOBAL, unsigned, int>;
+
 // Pairs of one slot's share [r0, r1) of the start list, r0 in bin b.  The buckets of the list are
 // (bin, clear starts), (bin, other starts) for every bin.  TEST: the series has NaN
 // between finite saves, so the partner is tested and the pairs counted.
-//
-// List positions are unsigned: a series may hold nearly 2^31 saves, and a position
-// runs up to a row past the end of the list.
 //
 // A pair that does not exist reads the start itself and adds (+0, 0): a select
 // on the address.  Predicates on the pair's arithmetic cost more (they become
@@ -275,10 +278,12 @@ __device__ __forceinline__ T start_sum(const T (&v)[NS], int q0, int j)
 template <typename MuT, typename IdxT, int NS, int MODE, bool TEST>
 __device__ __forceinline__ void dmumu_pairs(const MuT* series,
                                             const IdxT* list, const int* cur, bool clear_ok, int nb, int nl, int b,
-                                            unsigned r0, unsigned r1, int end_save, const unsigned (&off)[NS], int lane,
+                                            SavePos<MODE> r0, SavePos<MODE> r1, int end_save,
+                                            const unsigned (&off)[NS], int lane,
                                             const int* lane_lag, double* out_sd, double* out_sd2,
                                             unsigned long long* out_cnt, double* tot_sd2, int* tot_c)
 {
+    using Pos = SavePos<MODE>;
     constexpr unsigned kStride = slot_stride(MODE, sizeof(MuT));
     constexpr int kOwn = (NS + kStartLanes - 1) / kStartLanes, kShort = NS - long_sets(NS);
     const int j = lane / kLagLanes, l = lane % kLagLanes;
@@ -298,8 +303,8 @@ __device__ __forceinline__ void dmumu_pairs(const MuT* series,
     for (int k = 0; k < kOwn; ++k) own[k] = 0.0;
 #pragma unroll
     for (int k = 0; k < (TEST ? kOwn : 1); ++k) ownc[k] = 0;
-    for (unsigned e = r0; e < r1; ++b) {
-        const unsigned e1 = min((unsigned)cur[2 * b + 2], r1);
+    for (Pos e = r0; e < r1; ++b) {
+        const Pos e1 = min((Pos)cur[2 * b + 2], r1);
         if (e >= e1) continue;
         double sd[NS], sq[NS];
         int c[TEST ? NS : 1];
@@ -309,8 +314,7 @@ __device__ __forceinline__ void dmumu_pairs(const MuT* series,
         for (int k = 0; k < (TEST ? NS : 1); ++k) c[k] = 0;
         if constexpr (!TEST && MODE != SLOT_GLOBAL) {
             // whole rows of clear starts
-            const unsigned clear = min((unsigned)cur[2 * b + 1], e1);
-            const unsigned ec = clear_ok && clear > e ? e + ((clear - e) & ~(kStartLanes - 1u)) : e;
+            const Pos ec = clear_ok ? e + ((min((Pos)cur[2 * b + 1], e1) - e) & ~(kStartLanes - 1)) : e;
 #pragma unroll 2
             for (; e < ec; e += kStartLanes) {
                 const unsigned at = base + list[e + j] * kStride;
@@ -496,8 +500,8 @@ __global__ void __launch_bounds__(max_threads(NS), 1) dmumu_kernel(DmumuLaunch a
     }
     const MuT* mu = (const MuT*)a.mu;
     const int64_t step = (int64_t)gridDim.x * a.ppc, hop = T * a.ss;
-    // saves are unsigned where a loop runs past the last one: nsave may be nearly 2^31
-    const unsigned n_saves = (unsigned)nsave, clear_from = (unsigned)clear_end;
+    using Pos = SavePos<MODE>;
+    const Pos n_saves = (Pos)nsave, clear_from = (Pos)clear_end;
     for (int64_t p = cta * a.ppc + slot; p < a.n; p += step) {
         const MuT* row = mu + p * a.sp + st * a.ss;
         // ---- stage the series and count the starts per bucket, kBatch saves of a
@@ -507,14 +511,14 @@ __global__ void __launch_bounds__(max_threads(NS), 1) dmumu_kernel(DmumuLaunch a
         {
             int bad = nsave;
             const MuT* q = row;
-            auto stage = [&](unsigned s0, int (&b)[kBatch]) {
+            auto stage = [&](Pos s0, int (&b)[kBatch]) {
                 MuT v[kBatch];
 #pragma unroll
                 for (int i = 0; i < kBatch; ++i) v[i] = s0 + i * T < n_saves ? q[i * hop] : MuT(NAN);
                 bins_of(v, E, b);
 #pragma unroll
                 for (int i = 0; i < kBatch; ++i) {
-                    const unsigned s = s0 + i * T;
+                    const Pos s = s0 + i * T;
                     if (s < n_saves) {
                         const MuT x = b[i] >= 0 ? v[i] : MuT(NAN);
                         if constexpr (MODE == SLOT_REP) put_rep(series, s, x);
@@ -535,7 +539,7 @@ __global__ void __launch_bounds__(max_threads(NS), 1) dmumu_kernel(DmumuLaunch a
                     pk[i0 + i] = b[i] < 0 ? 0xffffffffu : (uint32_t)k << 16 | (uint32_t)atomicAdd(&hist[k], 1);
                 }
             }
-            for (unsigned s0 = kKeep * T + st; s0 < n_saves; s0 += kBatch * T) {
+            for (Pos s0 = kKeep * T + st; s0 < n_saves; s0 += kBatch * T) {
                 int b[kBatch];
                 stage(s0, b);
 #pragma unroll
@@ -584,12 +588,12 @@ __global__ void __launch_bounds__(max_threads(NS), 1) dmumu_kernel(DmumuLaunch a
                 list[cur[k] + (int)(pk[i] & 0xffffu)] = (IdxT)(i * T + st);
                 reach(i * T + st, k >> 1);
             }
-            for (unsigned s0 = kKeep * T + st; s0 < n_saves; s0 += kBatch * T) {
+            for (Pos s0 = kKeep * T + st; s0 < n_saves; s0 += kBatch * T) {
                 MuT v[kBatch];
                 int b[kBatch], at[kBatch];
 #pragma unroll
                 for (int i = 0; i < kBatch; ++i) {
-                    const unsigned s = s0 + i * T;
+                    const Pos s = s0 + i * T;
                     if constexpr (MODE == SLOT_REP)
                         v[i] = s < n_saves ? *(const MuT*)((const char*)series + 16 * (size_t)s) : MuT(NAN);
                     else
@@ -615,18 +619,18 @@ __global__ void __launch_bounds__(max_threads(NS), 1) dmumu_kernel(DmumuLaunch a
         // part of it)
         int bin0 = 0, bin1 = 0;
         auto boundary = [&](int k, int& b) {
-            const unsigned all = (unsigned)total + kFlushCost * (nb + 1);  // below 2^32
-            const unsigned target = (unsigned)(((unsigned long long)all * k) / a.parts);
+            const Pos all = (Pos)total + kFlushCost * (nb + 1);  // in 32 bits either way
+            const Pos target = (Pos)(((unsigned long long)all * k) / a.parts);
             b = 0;
             for (int hi = nb + 1; b + 1 < hi;) {
                 const int m = (b + hi) >> 1;
-                if ((unsigned)cur[2 * m] + kFlushCost * m <= target) b = m;
+                if ((Pos)cur[2 * m] + kFlushCost * m <= target) b = m;
                 else hi = m;
             }
             // the flushes up to b come before target: the chosen m passed that test
-            return min((unsigned)cur[2 * b + 2], max((unsigned)cur[2 * b], target - kFlushCost * b));
+            return min((Pos)cur[2 * b + 2], max((Pos)cur[2 * b], target - kFlushCost * b));
         };
-        const unsigned r0 = boundary(part, bin0), r1 = part + 1 == a.parts ? total : boundary(part + 1, bin1);
+        const Pos r0 = boundary(part, bin0), r1 = part + 1 == a.parts ? (Pos)total : boundary(part + 1, bin1);
         const int* lane_lag = s_lane + group * NS * kLagLanes;
         if (prefix)
             dmumu_pairs<MuT, IdxT, NS, MODE, false>(series, list, cur, nfin == nsave, nb, nl, bin0, r0, r1,
